@@ -409,41 +409,47 @@ __device__ void leg2(double *a, double *x, double *bb) {
   x[0] = bb[0] - a[1] * x[1];
 }
 
-// Dense solve with partial pivoting (ANM); returns false when singular.
-__device__ bool solve_pp(double *A, double *x, int m) {
+// Dense solve with partial pivoting (ANM) of order m <= 32 by one warp: lane i
+// owns row i of A (row stride ld) and x; false when singular or not finite.
+// Column k's pivot is the largest |A[i][k]|, the first of equals.
+__device__ bool solve_pp_warp(double *A, int ld, double *x, int m) {
+  const int lane = threadIdx.x & 31;
   for (int k = 0; k < m; ++k) {
-    int piv = k;
-    double best = fabs(A[k * m + k]);
-    for (int i = k + 1; i < m; ++i)
-      if (fabs(A[i * m + k]) > best) {
-        best = fabs(A[i * m + k]);
-        piv = i;
-      }
+    double best = lane >= k && lane < m ? fabs(A[lane * ld + k]) : -1.0;
+    if (!(best >= 0.0)) best = -1.0;  // NaN never pivots
+    int piv = lane;
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int op = __shfl_xor_sync(0xffffffffu, piv, o);
+      if (ob > best || (ob == best && op < piv)) best = ob, piv = op;
+    }
     if (!(best > 1e-300)) return false;
     if (piv != k) {
-      for (int j = 0; j < m; ++j) {
-        double tt = A[k * m + j];
-        A[k * m + j] = A[piv * m + j];
-        A[piv * m + j] = tt;
+      for (int j = lane; j <= m; j += 32) {
+        double *p = j < m ? A + k * ld + j : x + k, *q = j < m ? A + piv * ld + j : x + piv;
+        const double t = *p;
+        *p = *q;
+        *q = t;
       }
-      double tt = x[k];
-      x[k] = x[piv];
-      x[piv] = tt;
+      __syncwarp();
     }
-    for (int i = k + 1; i < m; ++i) {
-      double f = A[i * m + k] / A[k * m + k];
-      for (int j = k; j < m; ++j) A[i * m + j] -= f * A[k * m + j];
-      x[i] -= f * x[k];
+    if (lane > k && lane < m) {
+      const double f = A[lane * ld + k] / A[k * ld + k];
+      for (int j = k; j < m; ++j) A[lane * ld + j] -= f * A[k * ld + j];
+      x[lane] -= f * x[k];
     }
+    __syncwarp();
   }
+  bool fine = true;
   for (int k = m - 1; k >= 0; --k) {
-    double acc = x[k];
-    for (int j = k + 1; j < m; ++j) acc -= A[k * m + j] * x[j];
-    x[k] = acc / A[k * m + k];
+    const double xk = x[k] / A[k * ld + k];
+    fine = fine && isfinite(xk);
+    __syncwarp();
+    if (lane == k) x[k] = xk;
+    if (lane < k) x[lane] -= A[lane * ld + k] * xk;
+    __syncwarp();
   }
-  for (int k = 0; k < m; ++k)
-    if (!isfinite(x[k])) return false;
-  return true;
+  return fine;
 }
 
 // Reduce the IX partials of every solve: RMS and convergence/divergence
@@ -762,54 +768,57 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// ANM coefficients: update the ring Gram, solve for alpha (1 thread/solve).
-__global__ void k_anm_coef(const Desc *descs, const int *ctas, int force) {
+// ANM coefficients: update the ring Gram, solve for alpha (one CTA per solve).
+// A warp sums one dot's partials (lanes stride over the CTAs), one warp solves
+// the system in shared memory.  Latency-bound: one thread doing all of it took
+// 121 us of the 2.8 ms iteration at 256^3 with history 10.
+__global__ void __launch_bounds__(kThreads) k_anm_coef(const Desc *descs, const int *ctas) {
+  __shared__ double dot[kMaxHistory + 1], A[kMaxHistory * (kMaxHistory + 1)], x[kMaxHistory];
   const Desc &d = descs[blockIdx.x];
   Ctl *c = d.ctl;
-  if (threadIdx.x != 0) return;
   if (!c->mix_flag) return;
   const int nct = ctas[blockIdx.x];
-  const int H = d.history, H1 = H + 1, m = c->hcount;
-  double dot[kMaxHistory + 1];
-  for (int i = 0; i <= m; ++i) {
+  const int H = d.history, H1 = H + 1, m = c->hcount, head = c->hhead;
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x >> 5; i <= m; i += kThreads / 32) {
     double s = 0;
-    for (int k = 0; k < nct; ++k) s += d.partials[(size_t)k * kPartials + 1 + i];
-    dot[i] = s;
+    for (int k = lane; k < nct; k += 32) s += d.partials[(size_t)k * kPartials + 1 + i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) dot[i] = s;
   }
-  const int head = c->hhead;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
   // Gram rows of the newest residual (stored under the head slot)
-  c->gram[head * H1 + head] = dot[0];
-  int slot[kMaxHistory];
-  for (int i = 1; i <= m; ++i) {
-    slot[i - 1] = (head - i + 2 * H1) % H1;
-    c->gram[head * H1 + slot[i - 1]] = dot[i];
-    c->gram[slot[i - 1] * H1 + head] = dot[i];
-  }
-  double A[kMaxHistory * kMaxHistory], x[kMaxHistory];
+  auto slot = [&](int i) { return (head - 1 - i + 2 * H1) % H1; };
+  constexpr int LD = kMaxHistory + 1;
   const double Fkk = dot[0];
-  for (int i = 0; i < m; ++i) {
-    x[i] = Fkk - dot[i + 1];
+  if (lane == 0) c->gram[head * H1 + head] = Fkk;
+  if (lane < m) {
+    const int sl = slot(lane);
+    c->gram[head * H1 + sl] = dot[lane + 1];
+    c->gram[sl * H1 + head] = dot[lane + 1];
+    x[lane] = Fkk - dot[lane + 1];
     for (int j = 0; j < m; ++j)
-      A[i * m + j] = Fkk - dot[i + 1] - dot[j + 1] +
-                     c->gram[slot[i] * H1 + slot[j]];
+      A[lane * LD + j] = Fkk - dot[lane + 1] - dot[j + 1] + c->gram[sl * H1 + slot(j)];
   }
-  bool ok = m > 0 && solve_pp(A, x, m);
+  __syncwarp();
+  const bool ok = m > 0 && solve_pp_warp(A, LD, x, m);
+  __syncwarp();
+  if (lane < m) {
+    if (!ok) x[lane] = 0;
+    c->coef[1 + lane] = x[lane];
+    c->mix_slots[lane] = slot(lane);
+  }
+  __syncwarp();
+  if (lane != 0) return;
   double wsum = 0;
-  for (int i = 0; i < m; ++i) {
-    if (!ok) x[i] = 0;
-    wsum += x[i];
-  }
+  for (int i = 0; i < m; ++i) wsum += x[i];
   c->coef[0] = 1.0 - wsum;  // weight of the newest pair
-  for (int i = 0; i < m; ++i) {
-    c->coef[1 + i] = x[i];
-    c->mix_slots[i] = slot[i];
-  }
   c->mix_m = m;
   c->mix_head = head;
   // the newest pair joins the history
   c->hhead = (head + 1) % H1;
   if (c->hcount < H) c->hcount += 1;
-  (void)force;
 }
 
 // ANM mix: t_{k+1} = w_k (t_k + beta R_k) + sum_i alpha_i z_i ; the newest
@@ -1691,7 +1700,7 @@ void launch_anm(Batch b, int grid, const Desc *d, const int *ctas, int ns,
   if (stage == 0)
     k_anm_dots<P><<<grid, kThreads, 0, s>>>(b);
   else if (stage == 1)
-    k_anm_coef<<<ns, 32, 0, s>>>(d, ctas, 0);
+    k_anm_coef<<<ns, kThreads, 0, s>>>(d, ctas);
   else
     k_mix_anm<P><<<grid, kThreads, 0, s>>>(b);
 }
