@@ -130,7 +130,7 @@ template <typename P>
 void launch_anm(Batch, int, const Desc *, const int *, int, cudaStream_t, int);
 template <typename P>
 void launch_potential(const Desc &, const AtomTab &, double, double,
-                      const double *, int, double *, cudaStream_t);
+                      const double *, int, double, double *, cudaStream_t);
 void launch_phase_tables(double2 *, double2 *, double2 *, const double *,
                          const double *, const double *, int, int, int, int,
                          const double *, cudaStream_t);
@@ -1601,7 +1601,11 @@ static int init_typed(r3d_ctx *c, const ShellTable &st) {
     CK(cudaEventRecord(ev[0], s));
     if (nu > 0) {
       if (natom != (size_t)nu) return fail(c, R3D_EINVAL, "internal: atom stride");
-      launch_potential<P>(d, at, ikbt, ubeta, dr, coulomb, fr64, s);
+      // where the reference's clamps can act: r < 2e-3 sigma, r < 1e-5 A
+      // (with room for the rounding of r^2)
+      double rnear2 = 1.0e-9;
+      for (double s2 : sig2) rnear2 = std::max(rnear2, 4.1e-6 * s2);
+      launch_potential<P>(d, at, ikbt, ubeta, dr, coulomb, rnear2, fr64, s);
       CK(cudaGetLastError());
     } else {
       CK(cudaMemsetAsync(c->u, 0, n * N * sizeof(R), s));

@@ -983,6 +983,8 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int k = 0; k < kMixPer; ++k) {
     const long long i = i0 + k * kThreads;
+//   The sums kept are sum q/r and sum q e^{-r}/r: the short-range Coulomb part
+//   is the second, the long-range one their difference.
     if (i < niv) {
       rk[k] = res[i];
       zk[k] = (double)t[i] + beta * rk[k];
@@ -1036,12 +1038,42 @@ constexpr int kAtomTile = 128;
 // space (cal_Coulomb.cu:40-62); writes u[v] = beta u_LJ + q_v beta (phi -
 // phi_L), fr = beta phi_L(r), t0[v] = 0 (the short-range side of init_tuv's
 // t0 = q_v fr).
+        near = near || r2[j] < rnear2;
+      }
+      if (near) {  // a voxel all but on an atom: the reference's clamps
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+          const double i1 = rsqrt(r2[j]), i2 = i1 * i1, i6 = i2 * i2 * i2;
+#pragma unroll
+          for (int v = 0; v < M; ++v)
+            if (NS > 0 || v < n) {
+              const double s2 = at.sig2[v * at.nu + a0 + i], s6 = fmin(s2 * s2 * s2 * i6, smax6);
+              lj[j][v] = fma(at.eps4[v * at.nu + a0 + i], fma(s6, s6, -s6), lj[j][v]);
+            }
+          if (coulomb) {
+            if (r2[j] >= 1.0e-10) {  // r >= 1e-5 A
+              e[j] += azq.y * i1;
+              s[j] = fma(azq.y * i1, exp(-(r2[j] * i1)), s[j]);
+            } else {
+              s[j] -= azq.y;  // (1 - e^{-r}) / r -> 1
+            }
+          }
+        }
+        continue;
+      }
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
 //
 // The pair sums are the reference's, arranged so that one atom-voxel pair
-// costs one FP64 reciprocal square root and no division:
-//   1/r = rsqrt(r^2);  (sigma/r)^6 = sigma^6 (1/r^2)^3, clamped at 1/cut^6,
-//   which is the reference's clamp of (r/sigma)^2 from below at cut^2
-//   raised to the third power (four operations per site and pair);
+// costs one FP64 reciprocal square root and no division (the FP64 pipe bounds
+        ir12[j] = ir6[j] * ir6[j];
+// the kernel):
+//   1/r = rsqrt(r^2); 4 eps ((sigma/r)^12 - (sigma/r)^6) = A / r^12 - B / r^6
+//   with A = 4 eps sigma^12, B = 4 eps sigma^6 per atom and site: two
+//   operations per site and pair;
+//   the reference's clamp of (r/sigma)^2 from below at cut^2, and its r < 1e-5
+//   A case, can only act within r^2 < rnear2 (2e-3 of the largest sigma):
+//   such pairs take a branch of their own;
 //   e^{-r} of the long-range kernel (1 - e^{-r})/r is evaluated only for
 //   r <= 38 A: beyond, 1 - e^{-r} rounds to 1 in FP64, as it does in the
 //   reference, and most pairs of a protein-sized grid are that far apart.
@@ -1050,12 +1082,12 @@ constexpr int kAtomTile = 128;
 template <typename P, int NS, int V>
 __global__ void __launch_bounds__(kThreads)
     k_potential(Desc d, AtomTab at, double ikbt, double ubeta, double dx,
-                double dy, double dz, int coulomb, double *fr64) {
+                double dy, double dz, int coulomb, double rnear2, double *fr64) {
   using R = typename P::R;
   using T = typename P::T;
   constexpr int M = NS > 0 ? NS : kMaxSites;
   __shared__ double2 sxy[kAtomTile], szq[kAtomTile];
-  __shared__ double2 sse[M][kAtomTile];  // (sigma^6, 4 eps) per site
+  __shared__ double2 sab[M][kAtomTile];  // (A, B) per site
   const long long it = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = it * V < d.N;
   const long long ip = live ? it * V : 0;
@@ -1066,10 +1098,10 @@ __global__ void __launch_bounds__(kThreads)
   double rx[V];
 #pragma unroll
   for (int j = 0; j < V; ++j) rx[j] = (x + j - d.nx / 2) * dx;
-  double lj[V][M], e[V], f[V];
+  double lj[V][M], e[V], s[V];  // s: sum q e^{-r} / r
 #pragma unroll
   for (int j = 0; j < V; ++j) {
-    e[j] = f[j] = 0;
+    e[j] = s[j] = 0;
 #pragma unroll
     for (int v = 0; v < M; ++v) lj[j][v] = 0;
   }
@@ -1082,8 +1114,9 @@ __global__ void __launch_bounds__(kThreads)
       sxy[i] = make_double2(at.x[a0 + i], at.y[a0 + i]);
       szq[i] = make_double2(at.z[a0 + i], at.q[a0 + i]);
       for (int v = 0; v < n; ++v) {
-        const double s2 = at.sig2[v * at.nu + a0 + i];
-        sse[v][i] = make_double2(s2 * s2 * s2, at.eps4[v * at.nu + a0 + i]);
+        const double s2 = at.sig2[v * at.nu + a0 + i], s6 = s2 * s2 * s2;
+        const double b6 = at.eps4[v * at.nu + a0 + i] * s6;
+        sab[v][i] = make_double2(b6 * s6, b6);
       }
     }
     __syncthreads();
@@ -1091,7 +1124,8 @@ __global__ void __launch_bounds__(kThreads)
       const double2 axy = sxy[i], azq = szq[i];
       const double ddy = ry - axy.y, ddz = rz - azq.x;
       const double yz2 = fma(ddy, ddy, ddz * ddz);
-      double r2[V], ir[V], ir6[V];
+      double r2[V], ir[V], ir6[V], ir12[V];
+      bool near = false;
 #pragma unroll
       for (int j = 0; j < V; ++j) {
         const double ddx = rx[j] - axy.x;
@@ -1103,28 +1137,19 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
       for (int v = 0; v < M; ++v) {
         if (NS > 0 || v < n) {
-          const double2 se = sse[v][i];
+          const double2 ab = sab[v][i];
 #pragma unroll
-          for (int j = 0; j < V; ++j) {
-            const double s6 = fmin(se.x * ir6[j], smax6);
-            lj[j][v] = fma(se.y, fma(s6, s6, -s6), lj[j][v]);
-          }
+          for (int j = 0; j < V; ++j)
+            lj[j][v] = fma(ab.x, ir12[j], fma(-ab.y, ir6[j], lj[j][v]));
         }
       }
       if (coulomb) {
 #pragma unroll
         for (int j = 0; j < V; ++j) {
-          if (r2[j] >= 1.0e-10) {  // r >= 1e-5 A
-            const double qr = azq.y * ir[j];
-            const double ra = r2[j] * ir[j];
-            e[j] += qr;
-            if (ra <= 38.0)  // a branch, so that far pairs skip the exponential
-              f[j] = fma(qr, 1.0 - exp(-ra), f[j]);
-            else
-              f[j] += qr;  // = fma(qr, 1 - 0, f)
-          } else {
-            f[j] += azq.y;
-          }
+          const double qr = azq.y * ir[j], ra = r2[j] * ir[j];
+          e[j] += qr;
+          if (ra <= 38.0)  // a branch, so that far pairs skip the exponential
+            s[j] = fma(qr, exp(-ra), s[j]);
         }
       }
     }
@@ -1135,13 +1160,13 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int j = 0; j < V; ++j) {
     const long long q = ip + j;
-    const double bfr = f[j] * ubeta, bde = e[j] * ubeta;  // betar
+    const double bfr = (e[j] - s[j]) * ubeta, bsr = s[j] * ubeta;  // betar
     fr[q] = (R)bfr;
     if (fr64) fr64[q] = bfr;
 #pragma unroll
     for (int v = 0; v < M; ++v) {
       if (NS > 0 || v < n) {
-        u[(long long)v * d.Ns + q] = (R)(lj[j][v] * ikbt + d.qv[v] * bde - d.qv[v] * bfr);
+        u[(long long)v * d.Ns + q] = (R)(lj[j][v] * ikbt + d.qv[v] * bsr);
         t[(long long)v * d.Ns + q] = (T)0;
       }
     }
@@ -1707,14 +1732,14 @@ void launch_anm(Batch b, int grid, const Desc *d, const int *ctas, int ns,
 template <typename P>
 void launch_potential(const Desc &d, const AtomTab &at, double ikbt,
                       double ubeta, const double *dr, int coulomb,
-                      double *fr64, cudaStream_t s) {
+                      double rnear2, double *fr64, cudaStream_t s) {
   // two voxels per thread (nx is even); four measured 9% slower on a B200
   constexpr int V = 2;
   const long long thr = (d.N + V - 1) / V;
   int grid = (int)((thr + kThreads - 1) / kThreads);
 #define R3D_POT(NS)                                                           \
   k_potential<P, NS, V><<<grid, kThreads, 0, s>>>(d, at, ikbt, ubeta, dr[0], \
-                                                  dr[1], dr[2], coulomb, fr64)
+                                                  dr[1], dr[2], coulomb, rnear2, fr64)
   switch (d.n) {
     case 1: R3D_POT(1); break;
     case 2: R3D_POT(2); break;
@@ -1807,8 +1832,8 @@ void launch_set_short(const Desc &d, const double *src, void *dst,
   template void launch_anm<P>(Batch, int, const Desc *, const int *, int,      \
                               cudaStream_t, int);                              \
   template void launch_potential<P>(const Desc &, const AtomTab &, double,     \
-                                    double, const double *, int, double *,     \
-                                    cudaStream_t);                             \
+                                    double, const double *, int, double,       \
+                                    double *, cudaStream_t);                   \
   template void launch_cref<P>(const Desc &, double *, cudaStream_t);          \
   template void launch_lr_update<P>(const double *, void *, long long,         \
                                     cudaStream_t);                             \
