@@ -983,8 +983,6 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int k = 0; k < kMixPer; ++k) {
     const long long i = i0 + k * kThreads;
-//   The sums kept are sum q/r and sum q e^{-r}/r: the short-range Coulomb part
-//   is the second, the long-range one their difference.
     if (i < niv) {
       rk[k] = res[i];
       zk[k] = (double)t[i] + beta * rk[k];
@@ -1038,35 +1036,9 @@ constexpr int kAtomTile = 128;
 // space (cal_Coulomb.cu:40-62); writes u[v] = beta u_LJ + q_v beta (phi -
 // phi_L), fr = beta phi_L(r), t0[v] = 0 (the short-range side of init_tuv's
 // t0 = q_v fr).
-        near = near || r2[j] < rnear2;
-      }
-      if (near) {  // a voxel all but on an atom: the reference's clamps
-#pragma unroll
-        for (int j = 0; j < V; ++j) {
-          const double i1 = rsqrt(r2[j]), i2 = i1 * i1, i6 = i2 * i2 * i2;
-#pragma unroll
-          for (int v = 0; v < M; ++v)
-            if (NS > 0 || v < n) {
-              const double s2 = at.sig2[v * at.nu + a0 + i], s6 = fmin(s2 * s2 * s2 * i6, smax6);
-              lj[j][v] = fma(at.eps4[v * at.nu + a0 + i], fma(s6, s6, -s6), lj[j][v]);
-            }
-          if (coulomb) {
-            if (r2[j] >= 1.0e-10) {  // r >= 1e-5 A
-              e[j] += azq.y * i1;
-              s[j] = fma(azq.y * i1, exp(-(r2[j] * i1)), s[j]);
-            } else {
-              s[j] -= azq.y;  // (1 - e^{-r}) / r -> 1
-            }
-          }
-        }
-        continue;
-      }
-#pragma unroll
-      for (int j = 0; j < V; ++j) {
 //
 // The pair sums are the reference's, arranged so that one atom-voxel pair
 // costs one FP64 reciprocal square root and no division (the FP64 pipe bounds
-        ir12[j] = ir6[j] * ir6[j];
 // the kernel):
 //   1/r = rsqrt(r^2); 4 eps ((sigma/r)^12 - (sigma/r)^6) = A / r^12 - B / r^6
 //   with A = 4 eps sigma^12, B = 4 eps sigma^6 per atom and site: two
@@ -1077,6 +1049,8 @@ constexpr int kAtomTile = 128;
 //   e^{-r} of the long-range kernel (1 - e^{-r})/r is evaluated only for
 //   r <= 38 A: beyond, 1 - e^{-r} rounds to 1 in FP64, as it does in the
 //   reference, and most pairs of a protein-sized grid are that far apart.
+//   The sums kept are sum q/r and sum q e^{-r}/r: the short-range Coulomb part
+//   is the second, the long-range one their difference.
 // Each thread owns V voxels adjacent in x (nx a multiple of V), which share
 // an atom's y/z distance terms and its shared-memory loads.
 template <typename P, int NS, int V>
@@ -1130,9 +1104,35 @@ __global__ void __launch_bounds__(kThreads)
       for (int j = 0; j < V; ++j) {
         const double ddx = rx[j] - axy.x;
         r2[j] = fma(ddx, ddx, yz2);
+        near = near || r2[j] < rnear2;
+      }
+      if (near) {  // a voxel all but on an atom: the reference's clamps
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+          const double i1 = rsqrt(r2[j]), i2 = i1 * i1, i6 = i2 * i2 * i2;
+#pragma unroll
+          for (int v = 0; v < M; ++v)
+            if (NS > 0 || v < n) {
+              const double s2 = at.sig2[v * at.nu + a0 + i], s6 = fmin(s2 * s2 * s2 * i6, smax6);
+              lj[j][v] = fma(at.eps4[v * at.nu + a0 + i], fma(s6, s6, -s6), lj[j][v]);
+            }
+          if (coulomb) {
+            if (r2[j] >= 1.0e-10) {  // r >= 1e-5 A
+              e[j] += azq.y * i1;
+              s[j] = fma(azq.y * i1, exp(-(r2[j] * i1)), s[j]);
+            } else {
+              s[j] -= azq.y;  // (1 - e^{-r}) / r -> 1
+            }
+          }
+        }
+        continue;
+      }
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
         ir[j] = rsqrt(r2[j]);
         const double ir2 = ir[j] * ir[j];
         ir6[j] = ir2 * ir2 * ir2;
+        ir12[j] = ir6[j] * ir6[j];
       }
 #pragma unroll
       for (int v = 0; v < M; ++v) {
