@@ -121,6 +121,7 @@ template <typename P>
 void launch_inv_x(Batch, int, size_t, cudaStream_t, int, void *, int);
 void launch_reduce(const Desc *, const int *, int, int, cudaStream_t);
 void launch_ctl_gather(const Desc *, int, double *, cudaStream_t);
+int atom_chunks(int nu, long long N);
 void launch_atom_integrals(const IntAtoms &, const double *, long long, const int *,
                            const double *, double *, int, double *, cudaStream_t);
 template <typename P>
@@ -2427,7 +2428,16 @@ extern "C" int r3d_atom_integrals(r3d_ctx *c, double *grad, double *euv, double 
   else
     launch_gh<PMix>(d, tg, c->scratch, nullptr, s);
   const double lambda1 = p.adswitch == 1 ? p.lambda : 1.0;
-  std::vector<double> tab((size_t)nu * (4 + 2 * n));
+  std::vector<double> tab((size_t)nu * (4 + 4 * n));
+  // the smallest double whose square root is >= c (so that r^2 is compared
+  // exactly where sqrt(r^2) >= c was)
+  auto square_of = [](double c) {
+    if (!(c > 0)) return 0.0;  // every r qualifies
+    double t = c * c;
+    while (std::sqrt(t) >= c && t > 0) t = std::nextafter(t, -1.0);
+    while (std::sqrt(t) < c) t = std::nextafter(t, HUGE_VAL);
+    return t;
+  };
   for (int a = 0; a < nu; ++a) {
     tab[a] = p.r[3 * a];
     tab[nu + a] = p.r[3 * a + 1];
@@ -2436,9 +2446,12 @@ extern "C" int r3d_atom_integrals(r3d_ctx *c, double *grad, double *euv, double 
     for (int v = 0; v < n; ++v) {  // cal_LJ.cu:30-40
       tab[(size_t)(4 + v) * nu + a] = (p.sig[a] + p.sigv[v]) * 0.5 * lambda1;
       tab[(size_t)(4 + n + v) * nu + a] = std::sqrt(p.eps[a] * p.epsv[v]);
+      const double sg = tab[(size_t)(4 + v) * nu + a];
+      tab[(size_t)(4 + 2 * n + v) * nu + a] = square_of(sg * 0.5);
+      tab[(size_t)(4 + 3 * n + v) * nu + a] = square_of(sg * p.lambda * 0.5);
     }
   }
-  const int nchunk = (int)std::max<long long>(1, std::min<long long>(256, N / 4096));
+  const int nchunk = atom_chunks(nu, N);
   const long long nk = (long long)nu * (4 + n);
   double *buf = nullptr;
   const size_t bytes = (tab.size() + (size_t)nchunk * nk + nk) * sizeof(double);
@@ -2455,6 +2468,8 @@ extern "C" int r3d_atom_integrals(r3d_ctx *c, double *grad, double *euv, double 
     at.q = dtab + 3 * nu;
     at.sig = dtab + 4 * (size_t)nu;
     at.eps = dtab + (size_t)(4 + n) * nu;
+    at.cut2 = dtab + (size_t)(4 + 2 * n) * nu;
+    at.cutl2 = dtab + (size_t)(4 + 3 * n) * nu;
     for (int v = 0; v < n; ++v) {
       at.qv[v] = p.qv[v];
       at.rhov[v] = p.rhov[v];

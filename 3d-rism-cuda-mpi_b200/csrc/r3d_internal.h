@@ -182,6 +182,9 @@ constexpr int kPartials = 1 + 5 * kMaxSites;  // sum R^2 + per-site dots
 struct IntAtoms {
   const double *x, *y, *z, *q;  // [nu], device
   const double *sig, *eps;      // [n][nu], device: sigma_uv (with the LJ lambda), sqrt(eps_u eps_v)
+  // [n][nu], device: the smallest r^2 whose square root is >= sigma_uv / 2,
+  // and >= sigma_uv lambda / 2
+  const double *cut2, *cutl2;
   double qv[kMaxSites], rhov[kMaxSites];
   int nu, n, ad1;  // ad1: the LJ lambda derivative (else the Coulomb one)
   double lambda, cc;

@@ -1175,40 +1175,57 @@ __global__ void __launch_bounds__(kThreads)
 
 // ======================================================================
 // Post-solve per-atom integrals over g (cal_grad.cu:41-90, cal_euv.cu:29-65,
-// cal_ad1.cu, cal_ad2.cu), all atoms, sites and voxels in one launch: a CTA
-// takes one chunk of voxels and 256 atoms (one per thread); the chunk goes
-// through shared memory in tiles (g of every site and the voxel positions),
-// every thread sums its atom's terms over the tile, and the chunk's sums go
-// to partials [chunk][atom][k] that k_atom_reduce adds up.  Per atom
+// cal_ad1.cu, cal_ad2.cu), all atoms, sites and voxels in one launch.  Per atom
 // (k): 0-2 the force integrand sum_v rho_v g (24 eps s6 (2 s6 - 1) / r^2 +
 // q_u q_v cc / r^3) (x, y, z of voxel - atom), 3 the lambda derivative
 // (LJ: 24 eps s6 (2 s6 - 1) / lambda, r >= sigma lambda / 2; otherwise the
 // Coulomb term q_u q_v cc / r), 4.. the energy per site rho_v g (4 eps s6
 // (s6 - 1) + q_u q_v cc / r); terms only for r >= sigma_uv / 2.
+//
+// A CTA takes kIntAtoms atoms (one per lane, so 20 atoms use 20 of 32 lanes
+// and 300 waste 6 %) and one chunk of voxels, whose warps share the chunk's
+// tiles in shared memory (positions, rho_v g, and their charge density sum_v
+// q_v rho_v g); the warps' sums are added in warp order, the chunks' by
+// k_atom_reduce.  The FP64 pipe bounds it, so the pair work is sums of powers:
+// with w_v = rho_v g_v, an atom needs only sum w_v / r, sum w_v / r^6 and
+// sum w_v / r^12 per site (the energies and the lambda derivative are linear
+// in them) and the force from two site sums per pair -- one reciprocal square
+// root and no division, about 50 FP64 operations for four sites where the
+// formulas as written cost over 150.  Pairs closer than the largest cutoff of
+// the atom's sites (few voxels) are taken site by site.
 // ======================================================================
 constexpr int kIntTile = 256;  // voxels per shared-memory tile
+constexpr int kIntAtoms = 32;  // atoms per CTA
 
 template <int NS>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 2)
     k_atom_integrals(IntAtoms at, const double *g, long long N, int nx, int ny, int nz,
                      double dx, double dy, double dz, long long chunk, double *part) {
   constexpr int M = NS > 0 ? NS : kMaxSites;
-  __shared__ double sg[M][kIntTile];
-  __shared__ double sx[kIntTile], sy[kIntTile], sz[kIntTile];
+  constexpr int NW = kThreads / 32, K = 4 + M;
+  __shared__ double2 sxy[kIntTile], szq[kIntTile];  // (x, y), (z, charge density)
+  __shared__ double sw[M][kIntTile];                // rho_v g_v
   const int n = NS > 0 ? NS : at.n;
-  const int a = blockIdx.y * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int a = blockIdx.y * kIntAtoms + lane;
   const bool live = a < at.nu;
   const double ax = live ? at.x[a] : 0, ay = live ? at.y[a] : 0, az = live ? at.z[a] : 0;
-  const double qa = live ? at.q[a] : 0;
-  double sig[M], eps[M];
+  const double qa = live ? at.q[a] * at.cc : 0;
+  double c12[M], c6[M], near = 0;
 #pragma unroll
   for (int v = 0; v < M; ++v) {
-    sig[v] = (live && v < n) ? at.sig[v * at.nu + a] : 0;
-    eps[v] = (live && v < n) ? at.eps[v * at.nu + a] : 0;
+    c12[v] = c6[v] = 0;
+    if (live && v < n) {
+      const double sg = at.sig[v * at.nu + a], s2 = sg * sg, s6 = s2 * s2 * s2;
+      c6[v] = 24.0 * at.eps[v * at.nu + a] * s6;
+      c12[v] = 2.0 * c6[v] * s6;
+      near = fmax(near, fmax(at.cut2[v * at.nu + a], at.ad1 ? at.cutl2[v * at.nu + a] : 0.0));
+    }
   }
-  double fx = 0, fy = 0, fz = 0, ad = 0, e[M];
+  double fx = 0, fy = 0, fz = 0, adn = 0;      // adn: lambda derivative of the near pairs
+  double e1[M], e6[M], e12[M], en[M];          // en: energies of the near pairs
 #pragma unroll
-  for (int v = 0; v < M; ++v) e[v] = 0;
+  for (int v = 0; v < M; ++v) e1[v] = e6[v] = e12[v] = en[v] = 0;
   const long long c0 = blockIdx.x * chunk, c1 = min(N, c0 + chunk);
   for (long long t0 = c0; t0 < c1; t0 += kIntTile) {
     const int nt = (int)min((long long)kIntTile, c1 - t0);
@@ -1216,45 +1233,88 @@ __global__ void __launch_bounds__(kThreads)
     for (int i = threadIdx.x; i < nt; i += blockDim.x) {
       const long long ip = t0 + i;
       const int x = (int)(ip % nx), y = (int)((ip / nx) % ny), z = (int)(ip / ((long long)nx * ny));
-      sx[i] = (x - nx / 2) * dx;
-      sy[i] = (y - ny / 2) * dy;
-      sz[i] = (z - nz / 2) * dz;
-      for (int v = 0; v < n; ++v) sg[v][i] = g[(long long)v * N + ip];
+      double wq = 0;
+      for (int v = 0; v < n; ++v) {
+        const double w = at.rhov[v] * g[(long long)v * N + ip];
+        sw[v][i] = w;
+        wq += at.qv[v] * w;
+      }
+      sxy[i] = make_double2((x - nx / 2) * dx, (y - ny / 2) * dy);
+      szq[i] = make_double2((z - nz / 2) * dz, wq);
     }
     __syncthreads();
     if (!live) continue;
-    for (int i = 0; i < nt; ++i) {
-      const double ddx = sx[i] - ax, ddy = sy[i] - ay, ddz = sz[i] - az;
+    for (int i = warp; i < nt; i += NW) {
+      const double2 pxy = sxy[i], pzq = szq[i];
+      const double ddx = pxy.x - ax, ddy = pxy.y - ay, ddz = pzq.x - az;
       const double r2 = ddx * ddx + ddy * ddy + ddz * ddz;
-      const double r1 = sqrt(r2);
+      if (r2 >= near) {
+        const double ir = rsqrt(r2), ir2 = ir * ir, ir6 = ir2 * ir2 * ir2, ir12 = ir6 * ir6;
+        double s12 = 0, s6 = 0;
 #pragma unroll
-      for (int v = 0; v < M; ++v) {
-        if (NS == 0 && v >= n) break;
-        const double gv = sg[v][i];
-        const double qq = qa * at.qv[v] * at.cc;
-        const double s2 = sig[v] * sig[v] / r2, s6 = s2 * s2 * s2;
-        const double w = at.rhov[v] * gv;
-        if (r1 >= sig[v] * 0.5) {
-          const double fm = (eps[v] * 24.0 * s6 / r2 * (2.0 * s6 - 1.0) + qq / (r2 * r1)) * w;
-          fx += fm * ddx;
-          fy += fm * ddy;
-          fz += fm * ddz;
-          e[v] += (eps[v] * 4.0 * s6 * (s6 - 1.0) + qq / r1) * w;
-          if (!at.ad1) ad += qq / r1 * w;
+        for (int v = 0; v < M; ++v) {
+          if (NS == 0 && v >= n) break;
+          const double w = sw[v][i];
+          e1[v] = fma(w, ir, e1[v]);
+          e6[v] = fma(w, ir6, e6[v]);
+          e12[v] = fma(w, ir12, e12[v]);
+          s12 = fma(c12[v], w, s12);
+          s6 = fma(c6[v], w, s6);
         }
-        if (at.ad1 && r1 >= sig[v] * at.lambda * 0.5)
-          ad += eps[v] * 24.0 * s6 * (2.0 * s6 - 1.0) / at.lambda * w;
+        const double f = ir2 * fma(s12, ir12, fma(-s6, ir6, qa * pzq.y * ir));
+        fx = fma(f, ddx, fx);
+        fy = fma(f, ddy, fy);
+        fz = fma(f, ddz, fz);
+      } else {
+        const double ir = rsqrt(r2), ir2 = ir * ir, ir6 = ir2 * ir2 * ir2;
+        for (int v = 0; v < n; ++v) {
+          const double sg = at.sig[v * at.nu + a], sg2 = sg * sg, ep = at.eps[v * at.nu + a];
+          const double s6 = sg2 * sg2 * sg2 * ir6, w = sw[v][i], qi = qa * at.qv[v] * ir;
+          if (r2 >= at.cut2[v * at.nu + a]) {
+            const double f = (24.0 * ep * s6 * (2.0 * s6 - 1.0) + qi) * ir2 * w;
+            fx += f * ddx;
+            fy += f * ddy;
+            fz += f * ddz;
+            const double ev = (4.0 * ep * s6 * (s6 - 1.0) + qi) * w;
+#pragma unroll
+            for (int k = 0; k < M; ++k)
+              if (k == v) en[k] += ev;
+            if (!at.ad1) adn += qi * w;
+          }
+          if (at.ad1 && r2 >= at.cutl2[v * at.nu + a])
+            adn += 24.0 * ep * s6 * (2.0 * s6 - 1.0) / at.lambda * w;
+        }
       }
     }
   }
-  if (!live) return;
-  const int K = 4 + n;
-  double *o = part + ((long long)blockIdx.x * at.nu + a) * K;
-  o[0] = fx;
-  o[1] = fy;
-  o[2] = fz;
-  o[3] = ad;
-  for (int v = 0; v < n; ++v) o[4 + v] = e[v];
+  // this thread's K sums, then the warps' in warp order (through sw's space)
+  double o[K];
+  o[0] = fx, o[1] = fy, o[2] = fz, o[3] = adn;
+#pragma unroll
+  for (int v = 0; v < M; ++v) {
+    o[4 + v] = 0;
+    if (v < n) {
+      const double qq = qa * at.qv[v];
+      o[4 + v] = en[v] + (c12[v] * e12[v] / 12.0 - c6[v] * e6[v] / 6.0) + qq * e1[v];
+      o[3] += at.ad1 ? (c12[v] * e12[v] - c6[v] * e6[v]) / at.lambda : qq * e1[v];
+    }
+  }
+  __syncthreads();
+  double *red = &sw[0][0];  // [NW][32] of one sum at a time
+  static_assert(M * kIntTile >= NW * 32, "room for the warps' sums");
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (k >= 4 + n) break;
+    red[warp * 32 + lane] = o[k];
+    __syncthreads();
+    if (warp == 0 && live) {
+      double sum = 0;
+#pragma unroll
+      for (int j = 0; j < NW; ++j) sum += red[j * 32 + lane];
+      part[((long long)blockIdx.x * at.nu + a) * (4 + n) + k] = sum;
+    }
+    __syncthreads();
+  }
 }
 
 // out[a][k] = sum over the chunks of part[chunk][a][k]
@@ -1267,11 +1327,17 @@ __global__ void k_atom_reduce(const double *part, int nchunk, long long nk, doub
   }
 }
 
+// chunks of voxels: about four waves of CTAs over all atoms, 1024 voxels or
+// more each (a chunk costs every atom of its CTA a row of partial sums)
+int atom_chunks(int nu, long long N) {
+  const long long want = 148 * 2 * 4 / std::max(1, (nu + kIntAtoms - 1) / kIntAtoms) + 1;
+  return (int)std::max<long long>(1, std::min<long long>(std::max<long long>(want, 32), N / 1024));
+}
 void launch_atom_integrals(const IntAtoms &at, const double *g, long long N, const int *grid,
                            const double *dr, double *part, int nchunk, double *out,
                            cudaStream_t s) {
   const long long chunk = (N + nchunk - 1) / nchunk;
-  dim3 gr(nchunk, (at.nu + kThreads - 1) / kThreads);
+  dim3 gr(nchunk, (at.nu + kIntAtoms - 1) / kIntAtoms);
 #define R3D_INT(NS)                                                                      \
   k_atom_integrals<NS><<<gr, kThreads, 0, s>>>(at, g, N, grid[0], grid[1], grid[2], dr[0], \
                                                dr[1], dr[2], chunk, part)
