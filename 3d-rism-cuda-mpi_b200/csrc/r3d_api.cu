@@ -111,6 +111,32 @@ template <typename P>
 bool sr_launch_fx(int L, Batch b, int grid, size_t smem, cudaStream_t s);
 template <typename P>
 bool sr_launch_ix(int L, Batch b, int grid, size_t smem, cudaStream_t s, int per);
+// plane passes, any grid (r3d_passes_rt.cu)
+template <typename P>
+void rt_launch_fwd(const Desc &, Batch, int, int, size_t, cudaStream_t, int allow_mix);
+template <typename P>
+void rt_launch_inv(const Desc &, Batch, int, int, size_t, cudaStream_t, int mode);
+template <typename P>
+void rt_launch_y(const Desc &, int dir, Batch, int, size_t, cudaStream_t);
+template <typename P>
+void rt_launch_zoz(const Desc &, Batch, int, size_t, cudaStream_t);
+template <typename P>
+void rt_allow_fwd(const Desc &, int nt);
+template <typename P>
+int rt_allow_inv(const Desc &, int nt, size_t smem);
+template <typename P>
+void rt_allow_yz(const Desc &);
+bool rt_plan_axes(Desc &d, int kind);  // kind: 0 FP64, 1 FP32, 2 FP64 on FP32 grids
+bool rt_static_x(int kind, int nx, int ny, bool plane);
+bool rt_static_y(int kind, int ny);
+bool rt_listed(int n);
+int rt_threads(const Desc &d, int kind, int nsm);
+int rt_passes(int L, bool dbl);
+void launch_rt_reduce(const Desc *d, int ns, int mode, cudaStream_t s);
+void launch_mix_done(const Desc *d, cudaStream_t s);
+size_t rt_smem_x(int hx, int ny, int pr, bool plane, size_t csz);
+size_t rt_smem_y(int ny, int pc, size_t csz);
+size_t rt_smem_z(int nz, int n, int pc, size_t csz);
 template <typename P>
 void launch_fwd_x(Batch, int, size_t, cudaStream_t, int, const void *);
 template <typename P>
@@ -167,6 +193,8 @@ constexpr double hartree = 4.359744722207185e-18;
 constexpr size_t kSmemBudget = 100 * 1024;  // per CTA: two CTAs per SM
 constexpr size_t kSmemMax = 220 * 1024;
 constexpr int kNumSM = 148;
+// largest shared-memory plane of the plane passes
+constexpr size_t kRtPlaneMax = 92 * 1024;
 
 // resident CTAs per SM of a bulk-staged pass (device query; smem-only
 // estimate for host-only planning)
@@ -234,6 +262,10 @@ struct Geo {
   int mfx_avail = 0, mfx = 0, mfx_ctas = 0, mfx_per = 1;
   size_t smmfx = 0;
   size_t smx = 0, smy = 0, smz = 0;
+  // the plane passes (rt = 1: the iteration runs on them): CTAs per solve of
+  // the forward, y, z and inverse launches, their shared memory
+  int rt = 0, rt_dbl = 0, rt_nt = 256, rt_fctas = 0, rt_yctas = 0, rt_zctas = 0, rt_ictas = 0;
+  size_t rt_smx = 0, rt_smy = 0, rt_smz = 0;
 };
 
 struct r3d_ctx {
@@ -616,8 +648,36 @@ extern "C" int r3d_set_control(r3d_ctx *c, double convergence, int maxstep) {
 // ------------------------------------------------------------ geometry
 static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites);
 static bool ixb_config(int device, const Desc &d, bool fp64, int pcb, Geo &g);
+static bool plan_rt(int device, Desc &d, Geo &g, bool fp64);
+// Whether the mixed path's plane passes compute in FP64 on its FP32 grids and
+// spectra: the transforms' roundings are by far the largest in an iteration
+// (FP32 transforms are 3e-7 of h off, the spectra's storage 4e-8), and AN2
+// amplifies them from about the 15th iteration on, so g after 16 to 24
+// iterations comes out 2e-7 instead of 1e-6 to 1e-5 off.  It costs 5 to 15 % of
+// an iteration up to 96^3 (planes) and 40 % at 144^3 (275 us -> 391, four
+// sites).  Large grids, bound by their instructions, keep FP32 (256^3: 1.50 ms
+// an iteration against 2.08), and so do grids whose compile-time FP64 kernels
+// would take a pass more per axis (128^3: 198 us against 277).
+static bool rt_double(const Desc &d) {
+  if (d.N >= 3500000) return false;
+  if (!rt_listed(d.nx) || !rt_listed(d.ny) || !rt_listed(d.nz)) return true;
+  return rt_passes(d.hx, true) <= rt_passes(d.hx, false) &&
+         rt_passes(d.ny, true) <= rt_passes(d.ny, false) &&
+         rt_passes(d.nz, true) <= rt_passes(d.nz, false);
+}
+// Whether the iteration runs on the plane passes.  R3D_X_VARIANT=5 asks for
+// them, any other pinned variant (or a timing run of those) rules them out.
+static bool rt_wanted(const Desc &d, bool fp64) {
+  if (const char *ev = getenv("R3D_X_VARIANT")) return std::atoi(ev) == 5;
+  if (getenv("R3D_AUTOTUNE")) return false;
+  (void)d;
+  (void)fp64;
+  return true;
+}
 static int plan_geometry(r3d_ctx *c, Desc &d) {
-  return plan_geo(c, d, c->geo, c->fp64, c->prob.natv);
+  int rc = plan_geo(c, d, c->geo, c->fp64, c->prob.natv);
+  if (!rc) c->geo.rt = rt_wanted(d, c->fp64) && plan_rt(c->opts.device, d, c->geo, c->fp64);
+  return rc;
 }
 
 static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites) {
@@ -846,6 +906,86 @@ static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites) {
   return R3D_OK;
 }
 
+// ------------------------------------------------------------ plane passes
+// index whose transform value the engine leaves at position P
+static int rt_index_at(const RtPlan &p, int P) {
+  int K = 0, scale = 1;
+  for (int s = 0; s < p.n; ++s) {
+    const int u = P / p.m[s];
+    P -= u * p.m[s];
+    K += u * scale;
+    scale *= p.r[s];
+  }
+  return K;
+}
+
+// Launch geometry of the plane passes; false where they do not cover the
+// grid (a length with a prime factor over 13, more than four sites, an odd
+// nz).
+static bool plan_rt(int device, Desc &d, Geo &g, bool fp64) {
+  g.rt_dbl = !fp64 && rt_double(d);
+  const int kind = fp64 ? 0 : g.rt_dbl ? 2 : 1;
+  const size_t cs = kind == 1 ? 8 : 16;
+  if (device < 0 || d.n > 4 || (d.nz & 1)) return false;
+  auto magic = [](int v) { return v > 1 ? 0xffffffffu / (uint32_t)v + 1 : 0u; };
+  const int rows = d.ny * d.nz, V = !fp64 && d.hx % 2 == 0 ? 2 : 1;
+  // A whole plane per CTA (three launches an iteration) where two planes fit
+  // an SM with room to spare; else tiles of 32 rows (fewer for long rows) and
+  // y passes of their own (five).  Iterations of both on a B200, us, plane and
+  // tiles: 96^3, two sites, mixed 57 and 67; 144^3 147 and 189 (85 KB planes);
+  // 160^3 292 and 234 (105 KB: 320 planes over 296 places are two rounds);
+  // FP64, four sites, 96^3 (76 KB) 163 and 173; 120 x 100 x 84 (97 KB) 300 and
+  // 278; 144^3 (168 KB) 544 and 522.  Tiles too where they run kernels of
+  // compile-time sizes and the plane would not: 128 x 96 x 96, two sites, mixed
+  // 98 and 86, FP64 151 and 120.
+  d.rt_plane = rt_smem_x(d.hx, d.ny, d.ny, true, cs) <= kRtPlaneMax &&
+               (rt_static_x(kind, d.nx, d.ny, true) ||
+                !(rt_static_x(kind, d.nx, d.ny, false) && rt_static_y(kind, d.ny)));
+  if (!rt_plan_axes(d, kind)) return false;
+  d.rt_pr = d.rt_plane ? d.ny : 32;
+  while (!d.rt_plane && d.rt_pr > 4 && rt_smem_x(d.hx, d.ny, d.rt_pr, false, cs) > 72 * 1024)
+    d.rt_pr /= 2;
+  d.rt_pr = std::min(d.rt_pr, rows);
+  d.rt_tps = (rows + d.rt_pr - 1) / d.rt_pr;
+  d.rt_mghx = magic(d.hx);
+  d.rt_mghv = magic(d.hx / V);
+  d.rt_mgpr = magic(d.rt_pr);
+  d.rt_pcy = fp64 ? 8 : 16;
+  const int pcz = fp64 ? 4 : 8;
+  g.rt_smx = rt_smem_x(d.hx, d.ny, d.rt_pr, d.rt_plane != 0, cs);
+  g.rt_smy = rt_smem_y(d.ny, d.rt_pcy, cs);
+  g.rt_smz = rt_smem_z(d.nz, d.n, pcz, cs);
+  if (g.rt_smx > kSmemMax || g.rt_smy > kSmemMax || g.rt_smz > kSmemMax) return false;
+  g.rt_nt = rt_threads(d, kind, kNumSM);
+  int occ = 0;
+  if (fp64) {
+    rt_allow_fwd<P64>(d, g.rt_nt);
+    occ = rt_allow_inv<P64>(d, g.rt_nt, g.rt_smx);
+    rt_allow_yz<P64>(d);
+  } else if (g.rt_dbl) {
+    rt_allow_fwd<PMixD>(d, g.rt_nt);
+    occ = rt_allow_inv<PMixD>(d, g.rt_nt, g.rt_smx);
+    rt_allow_yz<PMixD>(d);
+  } else {
+    rt_allow_fwd<PMix>(d, g.rt_nt);
+    occ = rt_allow_inv<PMix>(d, g.rt_nt, g.rt_smx);
+    rt_allow_yz<PMix>(d);
+  }
+  if (occ < 1) return false;
+  d.rt_iper = 1;
+  d.rt_icps = d.rt_tps;
+  if (!d.rt_plane) {  // the inverse's sums: about one wave of CTAs
+    const int want = std::max(1, kNumSM * occ / d.n);
+    d.rt_iper = (d.rt_tps + want - 1) / want;
+    d.rt_icps = (d.rt_tps + d.rt_iper - 1) / d.rt_iper;
+  }
+  g.rt_fctas = d.n * d.rt_tps;
+  g.rt_ictas = d.n * d.rt_icps;
+  g.rt_yctas = d.rt_plane ? 0 : d.n * d.nz * ((d.hx + d.rt_pcy - 1) / d.rt_pcy);
+  g.rt_zctas = d.ny * ((d.hx + pcz - 1) / pcz);
+  return true;
+}
+
 // Geometry of the bulk-staged IX with pcb rows per tile (false: does not fit).
 static bool ixb_config(int device, const Desc &d, bool fp64, int pcb, Geo &g) {
   // rows per tile with compiled kernels: 8 or 4 (FP32 grids; 2 as well for
@@ -872,9 +1012,21 @@ static bool ixb_config(int device, const Desc &d, bool fp64, int pcb, Geo &g) {
 // descriptor (d.ct_* != 0), else on the runtime-length engine.
 // mode 1 with the mix-fused FX in use: allow_mix = 1 applies the mix the
 // last reduce requested (the iteration's graph), 0 is a plain FX (calculate)
+// f(the plane passes' types) of a geometry on precision P
+template <typename P, typename F>
+static void rt_typed(const Geo &g, F f) {
+  if (sizeof(typename P::R) == 4 && g.rt_dbl)
+    f(PMixD{});
+  else
+    f(P{});
+}
 template <typename P>
 static void pass_fx(const Desc &d, const Geo &g, Batch b, cudaStream_t s, int mode,
                     const void *src, int allow_mix = 0) {
+  if (mode == 1 && g.rt)
+    return rt_typed<P>(g, [&](auto q) {
+      rt_launch_fwd<decltype(q)>(d, b, g.rt_fctas, g.rt_nt, g.rt_smx, s, allow_mix);
+    });
   if (mode == 1 && g.mfx && ct_launch_mfx<P>(d.hx, b, g.mfx_ctas, g.smmfx, s, g.mfx_per, allow_mix))
     return;
   if (mode == 1 && g.fxs_pc && sr_launch_fx<P>(d.hx, b, g.fxs_ctas, g.smxs, s)) return;
@@ -898,7 +1050,12 @@ static void pass_zoz(const Desc &d, const Geo &g, Batch b, cudaStream_t s, int m
     launch_zoz<P>(b, g.tiles_z, g.smz, s, mode, check);
 }
 template <typename P>
-static void pass_ix(const Desc &d, const Geo &g, Batch b, cudaStream_t s, int mode, void *dst) {
+static void pass_ix(const Desc &d, const Geo &g, Batch b, cudaStream_t s, int mode, void *dst,
+                    int decide = 2) {
+  if (mode == 1 && g.rt)
+    return rt_typed<P>(g, [&](auto q) {
+      rt_launch_inv<decltype(q)>(d, b, g.rt_ictas, g.rt_nt, g.rt_smx, s, decide);
+    });
   if (mode == 1 && g.ixs_pc && sr_launch_ix<P>(d.hx, b, g.ixs_ctas, g.smxs, s, g.ixs_per)) return;
   if (mode == 1 && g.ixw_pc && ct_launch_xw<P>(1, d.hx, g.ixw_pc, b, g.ixw_ctas, g.smxw, s))
     return;
@@ -913,6 +1070,13 @@ static void pass_ix(const Desc &d, const Geo &g, Batch b, cudaStream_t s, int mo
 // else the tile-per-CTA kernels.
 template <typename P>
 static void pass_fy_iter(const Desc &d, const Geo &g, Batch b, cudaStream_t s, int dir) {
+  if (g.rt) {  // (a plane's y transform runs in its x pass)
+    if (!d.rt_plane)
+      rt_typed<P>(g, [&](auto q) {
+        rt_launch_y<decltype(q)>(d, dir, b, g.rt_yctas, g.rt_smy, s);
+      });
+    return;
+  }
   if (g.yz_tma >= 3 && sr_launch_fy<P>(d.ny, dir, b, g.fys_ctas, g.smfys, s)) return;
   if ((g.yz_tma == 1 || g.yz_tma == 2) &&
       tma_launch_fy<P>(d.ny, dir, b, g.fyt_ctas, g.smfyt, s, g.fyt_per, g.fyt_nst))
@@ -921,6 +1085,9 @@ static void pass_fy_iter(const Desc &d, const Geo &g, Batch b, cudaStream_t s, i
 }
 template <typename P>
 static void pass_zoz_iter(const Desc &d, const Geo &g, Batch b, cudaStream_t s) {
+  if (g.rt)
+    return rt_typed<P>(
+        g, [&](auto q) { rt_launch_zoz<decltype(q)>(d, b, g.rt_zctas, g.rt_smz, s); });
   if (g.yz_tma == 5 && g.yz_srp &&
       sr_launch_zozp<P>(d.nz, d.n, b, g.zs_ctas, g.zp_ctas, g.smzp, s))
     return;
@@ -934,18 +1101,18 @@ static void pass_zoz_iter(const Desc &d, const Geo &g, Batch b, cudaStream_t s) 
 
 // CTAs of the iteration's IX (each writes one row of the partials k_reduce sums)
 static int iter_ix_ctas(const Geo &g) {
-  return g.ixs_pc ? g.ixs_ctas : g.ixw_pc ? g.ixw_ctas : g.ixb_pc ? g.ixb_ctas : g.ix_ctas;
+  return g.rt ? g.rt_ictas : g.ixs_pc ? g.ixs_ctas : g.ixw_pc ? g.ixw_ctas : g.ixb_pc ? g.ixb_ctas : g.ix_ctas;
 }
 // rows of partials the iteration's IX may need, whichever variant runs
 static int max_ix_ctas(const Geo &g) {
   return std::max(std::max(std::max(std::max(g.ix_ctas, g.ixb_pc ? g.ixb_ctas : 0),
                                     g.ixw_pc ? g.ixw_ctas : 0),
                            g.ixh_ctas),
-                  g.ixs_pc ? g.ixs_ctas : 0);
+                  std::max(g.ixs_pc ? g.ixs_ctas : 0, g.rt ? g.rt_ictas : 0));
 }
 // CTAs of the iteration's FX
 static int iter_fx_ctas(const Geo &g) {
-  return g.mfx ? g.mfx_ctas : g.fxs_pc ? g.fxs_ctas : g.fxw_pc ? g.fxw_ctas
+  return g.rt ? g.rt_fctas : g.mfx ? g.mfx_ctas : g.fxs_pc ? g.fxs_ctas : g.fxw_pc ? g.fxw_ctas
                                       : g.fxb_pc ? g.fxb_ctas : g.tiles_x;
 }
 
@@ -961,8 +1128,8 @@ static int pf_len(int ns) { return PF_IXC * (ns + 1) + 2 * ns; }
 static std::vector<int> make_prefix(const Geo &g, int ns) {
   std::vector<int> v(pf_len(ns));
   const int per[6] = {iter_fx_ctas(g),
-                      g.yz_tma >= 3 ? g.fys_ctas : g.yz_tma ? g.fyt_ctas : g.tiles_y,
-                      g.yz_tma >= 3 ? g.zs_ctas : g.yz_tma == 2 ? g.zt_ctas : g.tiles_z,
+                      g.rt ? g.rt_yctas : g.yz_tma >= 3 ? g.fys_ctas : g.yz_tma ? g.fyt_ctas : g.tiles_y,
+                      g.rt ? g.rt_zctas : g.yz_tma >= 3 ? g.zs_ctas : g.yz_tma == 2 ? g.zt_ctas : g.tiles_z,
                       iter_ix_ctas(g), g.mix_ctas, g.dot_ctas};
   for (int k = 0; k < 6; ++k)
     for (int i = 0; i <= ns; ++i) v[pf_off(ns, k) + i] = i * per[k];
@@ -992,6 +1159,10 @@ static Geo scaled(const Geo &g, int ns) {
   s.mfx_ctas *= ns;
   s.mix_ctas *= ns;
   s.dot_ctas *= ns;
+  s.rt_fctas *= ns;
+  s.rt_yctas *= ns;
+  s.rt_zctas *= ns;
+  s.rt_ictas *= ns;
   return s;
 }
 
@@ -1072,6 +1243,20 @@ static int make_tmaps(r3d_ctx *c, Desc &d) {
   d.yrev = dy;
   d.tma_pc_y = g.fyt_pc;
   d.tma_pc_z = g.zt_pc;
+  return R3D_OK;
+}
+
+// k index at every position the plane passes leave digit-reversed
+static int make_rtrev(r3d_ctx *c, Desc &d) {
+  std::vector<int> v;
+  for (const RtPlan *p : {&d.rtx, &d.rty, &d.rtz})
+    for (int P = 0; P < p->L; ++P) v.push_back(rt_index_at(*p, P));
+  int *dv = nullptr;
+  int rc = dalloc(c, (void **)&dv, v.size() * sizeof(int));
+  if (rc) return rc;
+  CK(copy_h2d(c, dv, v.data(), v.size() * sizeof(int), c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  d.rtrev = dv;
   return R3D_OK;
 }
 
@@ -1260,6 +1445,10 @@ template <typename P>
 static int autotune_x(r3d_ctx *c) {
   Geo &g = c->geo;
   const Desc &d = c->desc;
+  if (g.rt) {  // the plane passes: no other variant
+    g.mfx = g.fxb_pc = g.ixb_pc = g.fxw_pc = g.ixw_pc = g.fxs_pc = g.ixs_pc = g.yz_tma = 0;
+    return R3D_OK;
+  }
   if (!g.fxb_pc && !g.ixb_pc && !g.fxw_pc && !g.ixw_pc && !g.fxs_pc && !g.yz_tma && !g.yz_sr)
     return R3D_OK;
   const std::array<int, 5> key{d.nx, d.ny, d.nz, d.n, c->fp64 ? 1 : 0};
@@ -1515,6 +1704,9 @@ static int init_typed(r3d_ctx *c, const ShellTable &st) {
   d.partials = c->partials;
   d.ctl = c->ctl;
   if ((rc = make_twiddles(c, d, c->fp64, &c->tw64, &c->tw32))) return rc;
+  if (c->geo.rt && (rc = make_rtrev(c, d))) return rc;
+  d.tw64 = c->tw64;
+  d.chi64 = c->fp64 ? c->chi : c->chi64;
   if ((rc = make_tmaps(c, d))) return rc;
   d.partial_base = 0;
   d.rmslog = rmslog;
@@ -1747,23 +1939,30 @@ static int enqueue_group(const Group &G, cudaStream_t s, int stage) {
     pass_fy_iter<P>(d, g, B(PF_Y), s, -1);
     pass_zoz_iter<P>(d, g, B(PF_Z), s);
     pass_fy_iter<P>(d, g, B(PF_Y), s, 1);
-    pass_ix<P>(d, g, B(PF_IX), s, 1, nullptr);
-    k += 5;
+    // the plane passes' inverse decides (reduces) in its last CTA, and their
+    // y transforms have no launch of their own in plane mode
+    pass_ix<P>(d, g, B(PF_IX), s, 1, nullptr, stage == 0 ? 0 : 2);
+    k += g.rt && d.rt_plane ? 3 : 5;
     if (G.mixer == MIX_ANM) {
       launch_anm<P>(B(PF_DOT), g.dot_ctas, G.ddescs, dotc, ns, s, 0);
       ++k;
     }
-    launch_reduce(G.ddescs, ixc, ns, stage == 0 ? 0 : 2, s);
-    ++k;
+    if (!g.rt) {
+      launch_reduce(G.ddescs, ixc, ns, stage == 0 ? 0 : 2, s);
+      ++k;
+    }
   } else {
-    launch_reduce(G.ddescs, ixc, ns, 1, s);
+    if (g.rt)
+      launch_rt_reduce(G.ddescs, ns, 1, s);
+    else
+      launch_reduce(G.ddescs, ixc, ns, 1, s);
     ++k;
   }
   if (stage != 1) {
     if (G.mixer == MIX_AN2) {
       // (with the mix-fused FX the iteration's mix runs at the start of the
       // next iteration's FX)
-      if (!(stage == 0 && g.mfx)) {
+      if (!(stage == 0 && (g.mfx || g.rt))) {
         launch_mix_an2<P>(B(PF_MIX), g.mix_ctas, s);
         ++k;
       }
@@ -1821,9 +2020,22 @@ extern "C" int r3d_anderson(r3d_ctx *c) {
     enqueue<P64>(c, 2);
   else
     enqueue<PMix>(c, 2);
+  // the mix has run: the plane passes' next iteration must not repeat it
+  if (c->geo.rt) launch_mix_done(c->ddesc, c->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->stream));
   return R3D_OK;
+}
+
+// FP64 on the plane passes: apply the mix that the last iteration requested
+// (the next iteration's forward pass would), so that t on the host is the t
+// of the start of the next iteration, as on the other FP64 paths.  (The mixed
+// path's fused passes have always left it pending.)
+static void flush_mix(r3d_ctx *c) {
+  if (!c->fp64 || !c->geo.rt || c->mixer != MIX_AN2) return;
+  const Group G = single_group(c);
+  launch_mix_an2<P64>(Batch{G.ddescs, G.dpf + pf_off(1, PF_MIX), 1}, G.geo.mix_ctas, c->stream);
+  launch_mix_done(c->ddesc, c->stream);
 }
 
 // One iteration captured once as a CUDA graph (pointers never change).
@@ -1867,6 +2079,7 @@ extern "C" int r3d_step(r3d_ctx *c, int nsteps, double *ms) {
   CK(cudaEventCreate(&e1));
   CK(cudaEventRecord(e0, c->stream));
   for (int i = 0; i < nsteps; ++i) CK(cudaGraphLaunch(c->gexec, c->stream));
+  flush_mix(c);
   CK(cudaEventRecord(e1, c->stream));
   CK(cudaEventSynchronize(e1));
   float t = 0;
@@ -1920,11 +2133,13 @@ static int profile_typed(r3d_ctx *c, int reps, std::string &names, double *ms,
     return R3D_OK;
   };
   const double cref = d.cref ? rs : 0.0;
-  if (c->geo.mfx) {
+  if (c->geo.mfx || (c->geo.rt && c->mixer == MIX_AN2)) {
     // the mix fused into FX: t, u, c_ref, and (mixing) the residual and the
     // four history rows in; t, its two history entries, g and w out
     const bool mixing = h.mix_flag != 0, picard = h.coef[2] < 0;
-    const double mixb = !mixing ? 0.0 : picard ? rs + ts + 2 * rs : 5 * rs + ts + 2 * rs;
+    const double mixb = !mixing ? 0.0
+                        : c->fp64 ? (picard ? rs + 2 * ts + rs : 3 * rs + 2 * ts + 2 * ts + rs)
+                        : picard ? rs + ts + 2 * rs : 5 * rs + ts + 2 * rs;
     timed("mix_fx", n * N * (ts + rs + cref + rs + ts + mixb),
           [&] { pass_fx<P>(d, c->geo, bx, s, 1, nullptr, 1); });
   } else {
@@ -1932,16 +2147,20 @@ static int profile_typed(r3d_ctx *c, int reps, std::string &names, double *ms,
     timed("fwd_x", n * N * (ts + rs + cref + rs + ts),
           [&] { pass_fx<P>(d, c->geo, bx, s, 1, nullptr); });
   }
-  timed("fft_y_fwd", n * N * 2 * rs,
-        [&] { pass_fy_iter<P>(d, c->geo, by, s, -1); });
+  const bool ypass = !(c->geo.rt && d.rt_plane);
+  if (ypass)
+    timed("fft_y_fwd", n * N * 2 * rs,
+          [&] { pass_fy_iter<P>(d, c->geo, by, s, -1); });
   timed("zoz", n * N * 2 * rs + (double)d.Nh * 4,
         [&] { pass_zoz_iter<P>(d, c->geo, bz, s); });
-  timed("fft_y_inv", n * N * 2 * rs,
-        [&] { pass_fy_iter<P>(d, c->geo, by, s, 1); });
+  if (ypass)
+    timed("fft_y_inv", n * N * 2 * rs,
+          [&] { pass_fy_iter<P>(d, c->geo, by, s, 1); });
   // IX: w, g, lr (and the two AN2 residual slots) in; R out
   timed("inv_x", n * N * (rs + ts + rs + rs + (dots ? 2 * rs : 0)),
         [&] { pass_ix<P>(d, c->geo, bix, s, 1, nullptr); });
-  if (c->mixer == MIX_AN2) {
+  if (c->mixer == MIX_AN2 && c->geo.rt) {  // reduced by inv_x, mixed by mix_fx
+  } else if (c->mixer == MIX_AN2) {
     timed("reduce", (double)iter_ix_ctas(c->geo) * kPartials * 8,
           [&] { launch_reduce(c->ddesc, ixc, 1, 1, s); });
     const bool picard = h.count_left > 0;
@@ -1953,8 +2172,9 @@ static int profile_typed(r3d_ctx *c, int reps, std::string &names, double *ms,
   } else {
     timed("anm_dots", n * N * rs * (h.hcount + 1),
           [&] { launch_anm<P>(bdot, c->geo.dot_ctas, c->ddesc, dotc, 1, s, 0); });
-    timed("reduce", (double)iter_ix_ctas(c->geo) * kPartials * 8,
-          [&] { launch_reduce(c->ddesc, ixc, 1, 1, s); });
+    if (!c->geo.rt)
+      timed("reduce", (double)iter_ix_ctas(c->geo) * kPartials * 8,
+            [&] { launch_reduce(c->ddesc, ixc, 1, 1, s); });
     timed("anm_coef", 0, [&] { launch_anm<P>(bmx, c->geo.mix_ctas, c->ddesc, dotc, 1, s, 1); });
     const int m = std::min(h.hcount, c->history);
     // FP64: R_k, t_k, m z entries in; R_k, z_k, t out.  Mixed: R_k, t_k, the
@@ -2047,9 +2267,10 @@ extern "C" int r3d_iterate(r3d_ctx *c, int *steps, double *rms, int *status) {
     for (int i = 0; i < chunk; ++i) CK(cudaGraphLaunch(c->gexec, s));
     int rc = read_ctl(c, h);
     if (rc) return rc;
-    if (ksave > 0 && h.status == RUNNING && h.step % ksave == 0 &&
-        (rc = r3d_write_tuv(c, nullptr)))
-      return rc;
+    if (ksave > 0 && h.status == RUNNING && h.step % ksave == 0) {
+      flush_mix(c);
+      if ((rc = r3d_write_tuv(c, nullptr))) return rc;
+    }
     if (!c->fp64 && h.status == RUNNING && h.rms < c->next_refresh) {
       // mixed path: move the converged part of c into the FP64 reference
       if ((rc = refresh<PMix>(c, false))) return rc;

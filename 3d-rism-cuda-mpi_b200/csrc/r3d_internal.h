@@ -75,17 +75,35 @@ std::string build_shells(const Problem &p, ShellTable &st);
 // FFT factor plan: radices outermost first.
 int factor_length(int L, int8_t *rad);
 
+// Passes of the run-time-planned engine (r3d_fft_rt.cuh) for one length:
+// radices r[0..n), m[s] the product of the radices after pass s, mg[s] its
+// division magic, tws[s] = L / (r[s] m[s]) the twiddle step of pass s.
+struct RtPlan {
+  int L, n;
+  int r[4], m[4], tws[4];
+  uint32_t mg[4];
+};
+
 // Precision of one solve: R = grid type (half spectra, u, L, residual and
 // residual history), T = state type (t and its mixing history).  The mixed
 // path keeps T in FP64: g = e^{t-u} multiplies any rounding of t by g (up to
 // ~30 at ion contact peaks), which an FP32 t would put at ~1e-5 in R.
+// A = arithmetic type of the plane passes' transforms and OZ (PMixD: FP64 on
+// FP32 grids and spectra, see r3d_passes_rt.cu).
 struct P64 {
   using R = double;
   using T = double;
+  using A = double;
 };
 struct PMix {
   using R = float;
   using T = double;
+  using A = float;
+};
+struct PMixD {
+  using R = float;
+  using T = double;
+  using A = double;
 };
 
 // ---------------------------------------------------------------------------
@@ -108,6 +126,7 @@ struct Ctl {
   int mix_m;                     // ANM: history entries used by this mix
   int mix_slots[kMaxHistory];    // ANM: their ring slots
   int err;                       // device-side error word
+  unsigned done;                 // k_rt_inv: CTAs whose sums are in
 };
 
 // Per-solve descriptor read by every pass kernel (device memory).
@@ -170,6 +189,16 @@ struct Desc {
   Tmap tm_y, tm_z;
   int tma_pc_y, tma_pc_z;
   const int *yrev;  // [ny]: ky index of each digit-reversed y row of w
+  // the plane passes (r3d_passes_rt.cu): plans, rows of an x tile (rt_plane:
+  // a whole z-plane, whose y transform runs in the same CTA), tiles per site,
+  // CTAs per site and tiles per CTA of the inverse, columns of a y tile,
+  // division magics (hx, hx / vector width, rows), k index at each
+  // digit-reversed position ([hx] of k_x, [ny] of k_y, [nz] of k_z)
+  RtPlan rtx, rty, rtz;
+  int rt_plane, rt_pr, rt_tps, rt_icps, rt_iper, rt_pcy;
+  uint32_t rt_mghx, rt_mghv, rt_mgpr;
+  const int *rtrev;
+  const void *tw64, *chi64;  // FP64 twiddles [twx pwx twy pwy twz pwz] and chi rows
   // polls of a staged pass's bounded wait for its copies before it gives up
   // (sets the error word); <= 0: the default, far beyond any copy's latency.
   // Set smaller only to exercise that error path (R3D_WAIT_POLLS).

@@ -41,6 +41,7 @@
 #include <stdint.h>
 
 #include "r3d_common.cuh"
+#include "r3d_reduce.cuh"
 
 namespace r3d {
 
@@ -397,18 +398,6 @@ __global__ void __launch_bounds__(kThreads)
 // ======================================================================
 // Control kernels (1 CTA per solve).
 // ======================================================================
-// leg (anderson.cu:105-130): 2x2 Gaussian elimination, no pivoting.
-__device__ void leg2(double *a, double *x, double *bb) {
-  double p = a[0];
-  a[1] /= p;
-  double r = bb[0] /= p;
-  double q = a[2];
-  a[3] -= q * a[1];
-  bb[1] -= q * r;
-  x[1] = bb[1] / a[3];
-  x[0] = bb[0] - a[1] * x[1];
-}
-
 // Dense solve with partial pivoting (ANM) of order m <= 32 by one warp: lane i
 // owns row i of A (row stride ld) and x; false when singular or not finite.
 // Column k's pivot is the largest |A[i][k]|, the first of equals.
@@ -492,62 +481,7 @@ __global__ void __launch_bounds__(kThreads)
   }
   __syncthreads();
   if (threadIdx.x != 0) return;
-  if (mode_force == 2) {  // calculate() only: record the rms, decide nothing
-    c->ss = sums[0];
-    c->rms = sqrt(sums[0] / ((double)d.N * d.n));
-    c->step += 1;
-    return;
-  }
-  if (mode_force == 0) {
-    c->ss = sums[0];
-    c->rms = sqrt(sums[0] / ((double)d.N * d.n));
-    c->step += 1;
-    if (c->step <= c->maxstep) d.rmslog[c->step - 1] = c->rms;
-    if (!isfinite(c->rms) || c->err) {  // err: a kernel's bounded wait ran out
-      c->status = DIVERGED;
-      c->mix_flag = 0;
-      return;
-    }
-    if (c->rms <= c->tol) {
-      c->status = CONVERGED;
-      c->mix_flag = 0;
-      return;
-    }
-    // The last allowed evaluation ends the solve without a mix: t stays the
-    // t of that evaluation, whose g and h the results are computed from.
-    if (c->step >= c->maxstep) {
-      c->status = MAXSTEP;
-      c->mix_flag = 0;
-      return;
-    }
-  }
-  c->mix_flag = 1;
-  if (d.mixer == MIX_AN2) {
-    if (c->count_left > 0) {  // newdt0 (Picard) step
-      c->count_left -= 1;
-      c->coef[0] = 0;
-      c->coef[1] = 0;
-      c->coef[2] = -1.0;  // marker: Picard
-      c->coef[3] = (double)c->binary;
-    } else {
-      double a[4], cc[2], x[2];
-      cc[0] = cc[1] = a[0] = a[1] = a[3] = 0.0;
-      for (int v = 0; v < d.n; ++v) {  // cal_theta, anderson.cu:81-102
-        cc[0] += sums[1 + 5 * v + 0] * d.irho[v];
-        cc[1] += sums[1 + 5 * v + 1] * d.irho[v];
-        a[0] += sums[1 + 5 * v + 2] * d.irho[v];
-        a[1] += sums[1 + 5 * v + 3] * d.irho[v];
-        a[3] += sums[1 + 5 * v + 4] * d.irho[v];
-      }
-      a[2] = a[1];
-      leg2(a, x, cc);
-      c->coef[0] = x[0] + d.mp * ((c->binary == 0) ? 0 : 1);
-      c->coef[1] = x[1] + d.mp * ((c->binary == 0) ? 1 : 0);
-      c->coef[2] = 1.0;
-      c->coef[3] = (double)c->binary;
-    }
-    c->binary = (c->binary == 0) ? 1 : 0;
-  }
+  reduce_finish(d, sums, mode_force);
 }
 
 // AN2 mix: newdt0 / newdt (anderson_cuda.cu:1-22), all sites in one launch.
@@ -1770,6 +1704,9 @@ __global__ void k_ctl_gather(const Desc *descs, int ns, double *out) {
 void launch_ctl_gather(const Desc *d, int ns, double *out, cudaStream_t s) {
   k_ctl_gather<<<(ns + kThreads - 1) / kThreads, kThreads, 0, s>>>(d, ns, out);
 }
+// The mix that the last reduce requested has been applied.
+__global__ void k_mix_done(const Desc *d) { d->ctl->mix_flag = 0; }
+void launch_mix_done(const Desc *d, cudaStream_t s) { k_mix_done<<<1, 1, 0, s>>>(d); }
 template <typename P>
 void launch_mix_an2(Batch b, int grid, cudaStream_t s) {
   k_mix_an2<P><<<grid, kThreads, 0, s>>>(b);
