@@ -164,6 +164,7 @@ void launch_phase_tables(double2 *, double2 *, double2 *, const double *,
 void launch_fk(const Desc &, double2 *, const double2 *, const double2 *,
                const double2 *, const double *, int, double, const double *,
                double, cudaStream_t);
+void launch_fk_physical(const Desc &, const double2 *, double2 *, double dv, cudaStream_t);
 template <typename P>
 void launch_cref(const Desc &, double *, cudaStream_t);
 template <typename P>
@@ -2342,12 +2343,35 @@ static int t_of_residual(r3d_ctx *c, const Ctl &h, const void **out) {
 // threads (which also share the first-touch page faults of a fresh
 // destination).  A direct pageable copy of a 256^3 x 4-site FP64 grid went
 // through the driver's own staging at a fraction of the link's rate.
+//
+// Page-locked destinations take the DMA directly (256^3 x 4 sites: 10 ms
+// against 20 through the staging; and a context that only ever copies to
+// such memory allocates no staging, 2 x 32 MB that take some 40 ms to
+// page-lock and to free).
 constexpr size_t kPinChunk = 32u << 20;
+static bool page_locked(const void *p, size_t bytes) {
+  auto locked = [](const void *q) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return a.type == cudaMemoryTypeHost;
+  };
+  return locked(p) && locked((const char *)p + bytes - 1);
+}
 static int copy_out(r3d_ctx *c, void *host, const void *dsrc, size_t bytes, cudaStream_t s) {
-  if (bytes < (4u << 20)) {  // small: one ordinary copy
-    CK(copy_d2h(c, host, dsrc, bytes, s));
-    CK(cudaStreamSynchronize(s));
-    return R3D_OK;
+  const bool small = bytes < (4u << 20);
+  if (small || page_locked(host, bytes)) {  // one ordinary copy
+    const cudaError_t e = copy_d2h(c, host, dsrc, bytes, s);
+    if (e == cudaSuccess) {
+      CK(cudaStreamSynchronize(s));
+      return R3D_OK;
+    }
+    // (a range whose ends are locked but not all of it: staged, as below)
+    if (small) CK(e);
+    cudaGetLastError();
+    c->d2h -= bytes;
   }
   for (int k = 0; k < 2; ++k) {
     if (!c->pin[k]) CK(cudaMallocHost(&c->pin[k], kPinChunk));
@@ -2514,7 +2538,13 @@ extern "C" int r3d_get_grid(r3d_ctx *c, int which, double *host) {
     case R3D_GRID_FK: case R3D_GRID_FKT: {
       count = 2 * d.Nh;
       if ((rc = ensure_scratch(c, count * 8))) return rc;
-      launch_to_double<P64>(c->fk, c->scratch, count, 0, s);  // FP64 always
+      if (which == R3D_GRID_FK) {  // transform units -> physical beta phi_L(k)
+        const Problem &p = c->prob;
+        launch_fk_physical(d, (const double2 *)c->fk, (double2 *)c->scratch,
+                           p.box[0] * p.box[1] * p.box[2] / (double)d.N, s);
+      } else {
+        launch_to_double<P64>(c->fk, c->scratch, count, 0, s);  // FP64 always
+      }
       break;
     }
     case R3D_GRID_CHI: {  // the shell table (FP64, times 2/N) through each point's shell
@@ -2535,19 +2565,6 @@ extern "C" int r3d_get_grid(r3d_ctx *c, int which, double *host) {
   }
   CK(cudaGetLastError());
   if ((rc = copy_out(c, host, c->scratch, count * 8, s))) return rc;
-  if (which == R3D_GRID_FK) {  // transform units -> physical beta phi_L(k)
-    const Problem &p = c->prob;
-    const double dv = p.box[0] * p.box[1] * p.box[2] / (double)d.N;
-    const int par0 = ((d.nx + d.ny + d.nz) / 2) & 1;
-    for (long long i = 0; i < d.Nh; ++i) {
-      int pp = (int)(i % d.hx), y = (int)((i / d.hx) % d.ny), z = (int)(i / ((long long)d.hx * d.ny));
-      double sg = ((2 * pp + y + z + par0) & 1) ? -1.0 : 1.0;
-      double a = host[2 * i], b = host[2 * i + 1];
-      // F = dv * C * raw, C = -i sigma:  (a + ib)(-i) = b - i a
-      host[2 * i] = dv * sg * b;
-      host[2 * i + 1] = -dv * sg * a;
-    }
-  }
   return R3D_OK;
 }
 

@@ -1408,6 +1408,20 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
 }
 
+// phi_L(k) from transform units to physical ones: times dv C(k), C(k) = -i
+// sigma, sigma = (-1)^{2p + y + z + (nx + ny + nz)/2}
+__global__ void k_fk_physical(Desc d, const double2 *fk, double2 *out, double dv) {
+  const int par0 = ((d.nx + d.ny + d.nz) / 2) & 1;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.Nh;
+       i += (long long)gridDim.x * blockDim.x) {
+    const int p = (int)(i % d.hx), y = (int)((i / d.hx) % d.ny),
+              z = (int)(i / ((long long)d.hx * d.ny));
+    const double sg = ((2 * p + y + z + par0) & 1) ? -1.0 : 1.0;
+    const double2 a = fk[i];
+    out[i] = make_double2(dv * sg * a.y, -dv * sg * a.x);  // (a + ib)(-i) = b - i a
+  }
+}
+
 // Refresh, step 1: freeze c_ref = c_s(t) in the grid type, and an FP64 copy
 // of exactly the stored values for the FP64 transform.
 template <typename P>
@@ -1766,6 +1780,10 @@ void launch_fk(const Desc &d, double2 *fk64, const double2 *ex,
   const long long tiles = (long long)((d.hx + kFkT - 1) / kFkT) * ((ncol + kFkT - 1) / kFkT);
   k_fk<<<(int)tiles, kThreads, 0, s>>>(d, fk64, ex, ey, ez, q, nu, ubeta, box[0],
                                        box[1], box[2], dv);
+}
+void launch_fk_physical(const Desc &d, const double2 *fk, double2 *out, double dv,
+                        cudaStream_t s) {
+  k_fk_physical<<<1184, kThreads, 0, s>>>(d, fk, out, dv);
 }
 template <typename P>
 void launch_cref(const Desc &d, double *c64, cudaStream_t s) {
