@@ -129,6 +129,7 @@ void rt_allow_yz(const Desc &);
 bool rt_plan_axes(Desc &d, int kind);  // kind: 0 FP64, 1 FP32, 2 FP64 on FP32 grids
 bool rt_static_x(int kind, int nx, int ny, bool plane);
 bool rt_static_y(int kind, int ny);
+bool rt_static_z(int kind, int nz, int n);
 bool rt_listed(int n);
 int rt_threads(const Desc &d, int kind, int nsm);
 int rt_passes(int L, bool dbl);
@@ -668,17 +669,41 @@ static bool rt_double(const Desc &d) {
 }
 // Whether the iteration runs on the plane passes.  R3D_X_VARIANT=5 asks for
 // them, any other pinned variant (or a timing run of those) rules them out.
-static bool rt_wanted(const Desc &d, bool fp64) {
+static bool rt_wanted() {
   if (const char *ev = getenv("R3D_X_VARIANT")) return std::atoi(ev) == 5;
-  if (getenv("R3D_AUTOTUNE")) return false;
-  (void)d;
-  (void)fp64;
-  return true;
+  return !getenv("R3D_AUTOTUNE");
+}
+// Whether the per-axis passes are the faster ones for a planned geometry: only
+// where they have compile-time-sized kernels on every axis and the plane passes
+// do not.  us per iteration, plane passes and per-axis passes:
+// - FP64 arithmetic on FP32 grids, planes in more than one round of two CTAs
+//   per SM, or tiles: four sites 80 x 72 x 96 134, 123; 64 x 72 x 80 107, 74;
+//   96 x 80 x 80 146, 123; 256 x 72 x 96 311, 222; 128 x 128 x 40 176, 110.
+//   In one round: 80 x 64 x 64 59, 79; two sites 80 x 72 x 96 56, 66.
+// - their rows of 24, 72 and 80 points (nx 48, 144, 160) are slow: four sites
+//   144 x 72 x 96 195, 236; 160 x 72 x 96 210, 224; 48 x 64 x 96 76, 80.
+// - 32^3: mixed four sites 37, 31, FP64 the same.
+// - FP64 grids, planes in more than one round, rows of 40 points or more:
+//   four sites 80 x 72 x 96 144, 137; 80 x 96 x 80 164, 153 (96 x 80 x 80 155,
+//   169); in two full rounds the plane passes: 80 x 72 x 128 164, 182.
+static bool per_axis_faster(const Desc &d, const Geo &g, bool fp64) {
+  const int kind = fp64 ? 0 : g.rt_dbl ? 2 : 1;
+  if (kind == 1 || !d.ct_x || !d.ct_y || !d.ct_z) return false;
+  if (rt_static_x(kind, d.nx, d.ny, d.rt_plane != 0) &&
+      (d.rt_plane || rt_static_y(kind, d.ny)) && rt_static_z(kind, d.nz, d.n))
+    return false;
+  const int planes = d.n * d.nz, round = 2 * kNumSM;
+  if (fp64)
+    return d.rt_plane && d.hx >= 40 && d.hx <= 48 && planes > round && 2 * planes < 3 * round;
+  return d.hx < 24 ||
+         (d.hx >= 32 && (d.hx <= 64 || d.hx == 128) && (!d.rt_plane || planes > round));
 }
 static int plan_geometry(r3d_ctx *c, Desc &d) {
   int rc = plan_geo(c, d, c->geo, c->fp64, c->prob.natv);
-  if (!rc) c->geo.rt = rt_wanted(d, c->fp64) && plan_rt(c->opts.device, d, c->geo, c->fp64);
-  return rc;
+  if (rc) return rc;
+  c->geo.rt = rt_wanted() && plan_rt(c->opts.device, d, c->geo, c->fp64);
+  if (c->geo.rt && !getenv("R3D_X_VARIANT") && per_axis_faster(d, c->geo, c->fp64)) c->geo.rt = 0;
+  return R3D_OK;
 }
 
 static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites) {
@@ -1399,8 +1424,9 @@ static size_t plan_bytes(const r3d_ctx *c, const Desc &d, int nshell) {
 // The iteration's x passes have two implementations each: one tile per CTA
 // with loads through registers (k_fx_ct / k_ix_ct), or persistent CTAs whose
 // inputs the bulk copy engine stages (k_fx_bulk / k_ix_bulk).  Which is
-// faster depends on the row length, the sites and the precision, so the
-// first solve of each geometry times both on its own buffers -- the mode-1 x
+// faster depends on the row length, the sites and the precision; with
+// R3D_AUTOTUNE=1 the first solve of each geometry times them on its own
+// buffers and prints what it took (a diagnostic) -- the mode-1 x
 // passes write only w, gq, the residual and the partials, which every
 // iteration rewrites -- and the choice holds for the process.
 static std::mutex g_tune_mu;
@@ -1408,27 +1434,16 @@ static std::mutex g_tune_mu;
 // 2 warp tiles, 3 (IX) bulk-staged with half-size tiles)
 static std::map<std::array<int, 5>, std::array<int, 3>> g_tune;  // + y/z on TMA
 
-// The committed choice per geometry.  Results of a solve depend (in their
-// last bits, which the Anderson iteration amplifies over hundreds of steps)
-// on the variant: each one sums the residual and its dots in its own order.
-// So the variant is a fixed function of the geometry -- this table, filled
-// from timings taken on a B200 with R3D_AUTOTUNE=1 (which times every
-// candidate and prints the row), else the rule in tune_rule -- and a solve
-// gives the same iterations and results on every box and every run.
-struct TuneRow {
-  int nx, ny, nz, n, fp64;
-  int fx, ix, yz;
-  int mfx;  // mixed AN2: 1 = the mix fused into FX (when the geometry has it)
-};
-static const TuneRow kTuneTable[] = {
-#include "r3d_tune_table.inc"
-};
-
-// Variants for a geometry with no row in the table (what the measured rows
-// favour): bulk-staged x passes for rows of 128 or more complex points, else
-// one tile per CTA (warp tiles for the shortest rows); the register-pass
-// Stockham y and z passes where they cover the lengths and sites, else the
-// copy-engine y passes with the tile-per-CTA z pass.
+// The choice per geometry, for the solves that the plane passes do not take.
+// Results of a solve depend (in their last bits, which the Anderson iteration
+// amplifies over hundreds of steps) on the variant: each one sums the residual
+// and its dots in its own order.  So the variant is a fixed function of the
+// geometry (tune_rule), and a solve gives the same iterations and results on
+// every GPU and every run; R3D_AUTOTUNE=1 times every candidate instead.
+// What the timings favour: bulk-staged x passes for rows of 128 or more complex
+// points, else one tile per CTA (warp tiles for the shortest rows); the
+// register-pass Stockham y and z passes where they cover the lengths and sites,
+// else the copy-engine y passes with the tile-per-CTA z pass.
 static std::array<int, 3> tune_rule(const Geo &g, const Desc &d) {
   std::array<int, 3> u{0, 0, 0};
   if (d.hx <= 32 && g.fxw_pc) u[0] = 2;
@@ -1470,23 +1485,9 @@ static int autotune_x(r3d_ctx *c) {
                         : (k == 1 && !d.ct_z) ? 0 : std::min(k, g.yz_tma);
     }
     known = true;
-  } else if (!getenv("R3D_AUTOTUNE")) {  // the committed table, else the fixed rule
+  } else if (!getenv("R3D_AUTOTUNE")) {
     use = tune_rule(g, d);
-    g.mfx = g.mfx_avail;  // the rule: fused where available
-    for (const TuneRow &r : kTuneTable)
-      if (r.nx == d.nx && r.ny == d.ny && r.nz == d.nz && r.n == d.n && r.fp64 == (c->fp64 ? 1 : 0)) {
-        use = {r.fx, r.ix, r.yz};
-        g.mfx = g.mfx_avail && r.mfx;
-        break;
-      }
-    // a row naming a variant this geometry does not offer falls back to the rule
-    const bool ok = (use[0] == 0 || (use[0] == 1 && g.fxb_pc) || (use[0] == 2 && g.fxw_pc) ||
-                     (use[0] == 4 && g.fxs_pc)) &&
-                    (use[1] == 0 || ((use[1] == 1 || use[1] == 3) && g.ixb_pc) ||
-                     (use[1] == 2 && g.ixw_pc) || (use[1] == 4 && g.ixs_pc)) &&
-                    (use[2] >= 3 ? (g.yz_sr && (use[2] <= 4 || (use[2] == 5 && g.yz_srp)))
-                                 : (use[2] <= g.yz_tma && !(use[2] == 1 && !d.ct_z)));
-    if (!ok) use = tune_rule(g, d);
+    g.mfx = g.mfx_avail;
     known = true;
   } else {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -2344,10 +2345,13 @@ static int t_of_residual(r3d_ctx *c, const Ctl &h, const void **out) {
 // destination).  A direct pageable copy of a 256^3 x 4-site FP64 grid went
 // through the driver's own staging at a fraction of the link's rate.
 //
-// Page-locked destinations take the DMA directly (256^3 x 4 sites: 10 ms
-// against 20 through the staging; and a context that only ever copies to
-// such memory allocates no staging, 2 x 32 MB that take some 40 ms to
-// page-lock and to free).
+// Page-locked destinations take the DMA directly: 256^3 x 4 sites 10 ms
+// against 20 through the staging, 95 MB 2.9 against 4.2; and a context that only
+// ever copies to such memory allocates no staging, 2 x 32 MB that take some
+// 40 ms to page-lock and to free.  A context that has its staging uses it for
+// what fits one chunk: a DMA into lines that the host's caches hold (a buffer
+// just made, or read since the last copy) runs at 8 GB/s (18 MB: 2.1 ms
+// against 1.1).
 constexpr size_t kPinChunk = 32u << 20;
 static bool page_locked(const void *p, size_t bytes) {
   auto locked = [](const void *q) {
@@ -2362,7 +2366,8 @@ static bool page_locked(const void *p, size_t bytes) {
 }
 static int copy_out(r3d_ctx *c, void *host, const void *dsrc, size_t bytes, cudaStream_t s) {
   const bool small = bytes < (4u << 20);
-  if (small || page_locked(host, bytes)) {  // one ordinary copy
+  const bool direct = !small && (!c->pin[0] || bytes > kPinChunk) && page_locked(host, bytes);
+  if (small || direct) {  // one ordinary copy
     const cudaError_t e = copy_d2h(c, host, dsrc, bytes, s);
     if (e == cudaSuccess) {
       CK(cudaStreamSynchronize(s));

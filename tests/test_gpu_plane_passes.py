@@ -191,3 +191,32 @@ def test_grid_copy_to_page_locked_memory(tmp_path, solvents):
         assert rc == 0
         assert np.array_equal(buf.numpy(), np.ascontiguousarray(ref).view(np.float64).reshape(-1))
     s.close()
+
+
+# the rule that leaves a geometry to the per-axis passes: a default solve is
+# the pinned plane-pass solve where it does not apply, and close to it where it
+# does (more than one round of planes; tiles; the shortest rows)
+@pytest.mark.parametrize("precision,n,dims,plane", [
+    ("mixed", 4, (64, 72, 80), False), ("mixed", 4, (80, 64, 64), True),
+    ("mixed", 2, (128, 128, 40), False), ("mixed", 2, (32, 32, 32), False),
+    ("mixed", 2, (48, 48, 40), True), ("fp64", 4, (80, 72, 80), False),
+    ("fp64", 4, (64, 72, 80), True)])
+def test_default_passes_by_geometry(tmp_path, monkeypatch, solvents, precision, n, dims, plane):
+    import rism3d as R
+    import synthetic as S
+    xvk = solvents["h2o_vv" if n == 2 else "naclaq_vv"]
+    inp = S.small(str(tmp_path), nu=12, grid=dims, box=tuple(0.5 * k for k in dims), solvent=xvk, seed=3)
+    out = []
+    for variant in (None, "5"):
+        if variant:
+            monkeypatch.setenv("R3D_X_VARIANT", variant)
+        s = R.RISM3D(precision=precision)
+        s.load(inp, xvk=xvk)
+        s.initialize()
+        s.step(4)
+        out.append(s.get("g"))
+        s.close()
+    same = np.array_equal(out[0], out[1])
+    assert same == plane
+    # four iterations' roundings: FP32 spectra 1e-5 of the largest g, FP64 1e-10
+    assert np.abs(out[0] - out[1]).max() <= (1e-5 if precision == "mixed" else 1e-10) * np.abs(out[1]).max()
