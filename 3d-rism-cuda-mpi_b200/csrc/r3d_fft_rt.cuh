@@ -203,9 +203,10 @@ __device__ __forceinline__ void rt_pass(int W, uint32_t mgW, int L, int M, uint3
 
 // Pass s of a length.  LS > 0: the length is a template constant and s an
 // integral_constant, so that the plan, every stride and every division fold;
-// LS = 0: plan p, s an int.
-template <int LS, int DIR, int NT, int RM, typename S, typename C, typename Ld, typename St>
-__device__ __forceinline__ void rt_pass_s(const RtPlan &p, S sc, int W, uint32_t mgW, const C *tw,
+// LS = 0: plan p (RtPlan's members, of any length), s an int.
+template <int LS, int DIR, int NT, int RM, typename PL, typename S, typename C, typename Ld,
+          typename St>
+__device__ __forceinline__ void rt_pass_s(const PL &p, S sc, int W, uint32_t mgW, const C *tw,
                                           Ld ld, St st) {
   if constexpr (LS > 0) {
     constexpr RtPlan pl = rt_plan_of(LS, RM);

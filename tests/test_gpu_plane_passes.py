@@ -102,14 +102,34 @@ def test_fp64_step_leaves_the_mixed_t(tmp_path, monkeypatch, solvents, n):
     assert out["5"][2] == out["0"][2] == n + 2
 
 
-@pytest.mark.parametrize("n,nz,ny,nx", [(1, 6, 10, 22), (3, 4, 1, 6), (2, 1, 13, 8), (2, 14, 35, 52)])
+class _ReducedPhases:
+    """The dense stages' matrices with every phase reduced to one turn in whole
+    numbers first: unreduced, phases of up to 2 pi 9000 are 7e-12 off."""
+
+    @staticmethod
+    def _mx(nx):
+        x, p = np.arange(nx), np.arange(nx // 2)
+        return ((-1.0) ** x)[None, :] * np.exp(-1j * np.pi * (np.outer(4 * p + 1, x) % (2 * nx)) / nx)
+
+    @staticmethod
+    def _mk(n):
+        j = np.arange(n)
+        return np.exp(-1j * np.pi * (np.outer(2 * j + 1, j) % (2 * n)) / n)
+
+
+# (4 and 9000: the shortest and about the longest row; 3125: five passes)
+@pytest.mark.parametrize("n,nz,ny,nx", [(1, 6, 10, 22), (3, 4, 1, 6), (2, 1, 13, 8), (2, 14, 35, 52),
+                                        (1, 4, 6, 4), (1, 2, 3125, 4), (1, 2, 2, 9000)])
 def test_slab_stages_match_numpy(n, nz, ny, nx):
     import torch
     import rism3d as R
     import slabs
     rng = np.random.default_rng(nx)
     real = rng.standard_normal((n, nz, ny, nx))
-    np_st, cu = slabs.NumpyStages(), slabs.CudaStages(R.lib, 0)
+    class Stages(_ReducedPhases, slabs.NumpyStages):
+        pass
+
+    np_st, cu = Stages(), slabs.CudaStages(R.lib, 0)
     ref = np.stack([np_st.forward_z(np_st.forward_xy(real[v])) for v in range(n)])
     spec = cu.forward_z_all(cu.forward_xy_all(torch.from_numpy(real).cuda()))
     got = torch.view_as_complex(spec.contiguous()).cpu().numpy()
