@@ -2346,12 +2346,12 @@ static int t_of_residual(r3d_ctx *c, const Ctl &h, const void **out) {
 // through the driver's own staging at a fraction of the link's rate.
 //
 // Page-locked destinations take the DMA directly: 256^3 x 4 sites 10 ms
-// against 20 through the staging, 95 MB 2.9 against 4.2; and a context that only
-// ever copies to such memory allocates no staging, 2 x 32 MB that take some
-// 40 ms to page-lock and to free.  A context that has its staging uses it for
-// what fits one chunk: a DMA into lines that the host's caches hold (a buffer
-// just made, or read since the last copy) runs at 8 GB/s (18 MB: 2.1 ms
-// against 1.1).
+// against 20 through the staging, 95 MB 2.9 against 4.2, 18 MB 0.4 against 1.1;
+// a pass over a screen of twelve solves, grids read back, 19 ms against 59; and a
+// context that only ever copies to such memory allocates no staging, 2 x 32 MB
+// that take some 40 ms to page-lock and to free.  (A buffer whose lines the
+// host's caches hold, just made or read since the last copy, takes the DMA at
+// 8 GB/s: 18 MB 2.1 ms.)
 constexpr size_t kPinChunk = 32u << 20;
 static bool page_locked(const void *p, size_t bytes) {
   auto locked = [](const void *q) {
@@ -2366,8 +2366,7 @@ static bool page_locked(const void *p, size_t bytes) {
 }
 static int copy_out(r3d_ctx *c, void *host, const void *dsrc, size_t bytes, cudaStream_t s) {
   const bool small = bytes < (4u << 20);
-  const bool direct = !small && (!c->pin[0] || bytes > kPinChunk) && page_locked(host, bytes);
-  if (small || direct) {  // one ordinary copy
+  if (small || page_locked(host, bytes)) {  // one ordinary copy
     const cudaError_t e = copy_d2h(c, host, dsrc, bytes, s);
     if (e == cudaSuccess) {
       CK(cudaStreamSynchronize(s));
