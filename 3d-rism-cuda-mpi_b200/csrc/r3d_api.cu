@@ -2937,10 +2937,22 @@ extern "C" int r3d_fft3d(int device, int precision, int nx, int ny, int nz,
 
 // ----------------------------------------------------------------- batches
 // Independent solves iterated together: the solves of one geometry (grid,
-// sites, mixer) form a group, each kernel of an iteration covers every solve
+// sites, mixer, passes) form a group, each kernel of an iteration covers every solve
 // of its group (a CTA finds its solve in the group's prefix block), and one
 // CUDA graph holds one iteration of all groups.  Solves that have converged,
 // diverged or hit maxstep are skipped by every kernel while the others run.
+// Contexts that one launch may cover: the launch takes its geometry and
+// kernels from the first of them and each solve's descriptor supplies the
+// rest, so all must have been planned alike.  The per-axis variants share one
+// descriptor layout; the plane passes' plans, tables and tile counts are in
+// the descriptors planned for them alone (geo.rt, which R3D_X_VARIANT,
+// R3D_AUTOTUNE and the like at r3d_initialize decide, not the shape alone).
+using GroupKey = std::array<long long, 7>;
+static GroupKey group_key(const r3d_ctx *c) {
+  return {c->desc.nx, c->desc.ny, c->desc.nz, c->desc.n, c->mixer,
+          c->mixer == MIX_ANM ? c->history : 0, c->geo.rt};
+}
+
 struct r3d_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -3021,11 +3033,9 @@ template <typename P>
 static int batch_build(r3d_batch *b) {
   batch_release(b);
   std::vector<std::vector<int>> members;
-  std::vector<std::array<long long, 6>> keys;
+  std::vector<GroupKey> keys;
   for (int i = 0; i < (int)b->ctxs.size(); ++i) {
-    const r3d_ctx *c = b->ctxs[i];
-    const std::array<long long, 6> key{c->desc.nx, c->desc.ny, c->desc.nz, c->desc.n,
-                                       c->mixer, c->mixer == MIX_ANM ? c->history : 0};
+    const GroupKey key = group_key(b->ctxs[i]);
     size_t g = std::find(keys.begin(), keys.end(), key) - keys.begin();
     if (g == keys.size()) {
       keys.push_back(key);

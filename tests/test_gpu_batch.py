@@ -94,6 +94,36 @@ def test_batch_rejects_bad_members(refcase):
 
 
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_contexts_of_different_passes_form_their_own_groups(refcase, monkeypatch, prec):
+    """One launch covers only contexts planned alike: a solve pinned to the
+    per-axis passes and one on the plane passes share a batch but no group,
+    and each ends where it ends alone."""
+    import rism3d as R
+    ctxs, solo = [], []
+    for k in range(2):
+        for variant in ("0", "5"):
+            monkeypatch.setenv("R3D_X_VARIANT", variant)
+            s = _make(R, refcase, "s64nacl", None, prec)
+            if k == 0:
+                solo.append((s.iterate(), s.get("g")))
+                s.close()
+            else:
+                ctxs.append(s)
+    b = R.Batch()
+    for s in ctxs:
+        b.add(s)
+    b.iterate()
+    assert b.info()["groups"] == 2
+    for s, (st, g) in zip(ctxs, solo):
+        steps, rms, status = s.status()
+        assert (steps, status) == (st[0], st[2])
+        assert np.array_equal(s.get("g"), g)
+    b.close()
+    for s in ctxs:
+        s.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
 def test_48_grid_matches_oracle_and_batches(solvents, tmp_path, prec):
     """48^3 cells (the smallest grid the batched screen's configuration
     names, which its solute-plus-buffer rule never reaches): two small
