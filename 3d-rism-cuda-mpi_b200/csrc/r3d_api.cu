@@ -2029,14 +2029,17 @@ extern "C" int r3d_anderson(r3d_ctx *c) {
   return R3D_OK;
 }
 
-// FP64 on the plane passes: apply the mix that the last iteration requested
-// (the next iteration's forward pass would), so that t on the host is the t
-// of the start of the next iteration, as on the other FP64 paths.  (The mixed
-// path's fused passes have always left it pending.)
+// Apply the mix that the last iteration requested, where the next iteration's
+// forward pass would (the plane passes, the mix-fused FX), so that t on the
+// host is the t of the start of the next iteration, as on the other paths.
 static void flush_mix(r3d_ctx *c) {
-  if (!c->fp64 || !c->geo.rt || c->mixer != MIX_AN2) return;
+  if (!(c->geo.rt || c->geo.mfx) || c->mixer != MIX_AN2) return;
   const Group G = single_group(c);
-  launch_mix_an2<P64>(Batch{G.ddescs, G.dpf + pf_off(1, PF_MIX), 1}, G.geo.mix_ctas, c->stream);
+  const Batch b{G.ddescs, G.dpf + pf_off(1, PF_MIX), 1};
+  if (c->fp64)
+    launch_mix_an2<P64>(b, G.geo.mix_ctas, c->stream);
+  else
+    launch_mix_an2<PMix>(b, G.geo.mix_ctas, c->stream);
   launch_mix_done(c->ddesc, c->stream);
 }
 
