@@ -2022,8 +2022,8 @@ extern "C" int r3d_anderson(r3d_ctx *c) {
     enqueue<P64>(c, 2);
   else
     enqueue<PMix>(c, 2);
-  // the mix has run: the plane passes' next iteration must not repeat it
-  if (c->geo.rt) launch_mix_done(c->ddesc, c->stream);
+  // the mix has run: a forward pass that mixes must not repeat it
+  if (c->geo.rt || c->geo.mfx) launch_mix_done(c->ddesc, c->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->stream));
   return R3D_OK;

@@ -152,6 +152,15 @@ def test_step_applies_the_pending_mix(tmp_path, monkeypatch, solvents, prec, pat
     _same_sequence(R, monkeypatch, tmp_path, solvents["h2o_vv"], prec, path, ops)
 
 
+@pytest.mark.parametrize("path", sorted(DEFERRED))
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_step_after_anderson_mixes_once(tmp_path, monkeypatch, solvents, prec, path):
+    """The mix that r3d_anderson has applied is not pending any more."""
+    import rism3d as R
+    _same_sequence(R, monkeypatch, tmp_path, solvents["h2o_vv"], prec, path,
+                   ("calculate", "anderson", 1, 1))
+
+
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 def test_ksave_file_holds_the_mixed_t(tmp_path, monkeypatch, solvents, prec):
     """The .tuv that iterate saves after step 3 is the t of the start of step 4."""
