@@ -668,10 +668,11 @@ static bool rt_double(const Desc &d) {
          rt_passes(d.nz, true) <= rt_passes(d.nz, false);
 }
 // Whether the iteration runs on the plane passes.  R3D_X_VARIANT=5 asks for
-// them, any other pinned variant (or a timing run of those) rules them out.
+// them; any other pinned variant (or a timing run of those) rules them out, and
+// so does R3D_MFX, which pins a form of the per-axis passes.
 static bool rt_wanted() {
   if (const char *ev = getenv("R3D_X_VARIANT")) return std::atoi(ev) == 5;
-  return !getenv("R3D_AUTOTUNE");
+  return !getenv("R3D_AUTOTUNE") && !getenv("R3D_MFX");
 }
 // Whether the per-axis passes are the faster ones for a planned geometry: only
 // where they have compile-time-sized kernels on every axis and the plane passes

@@ -81,3 +81,21 @@ def test_yz_pass_variant_matches_reference(refcase, tmp_path, monkeypatch, yz, c
         else:
             assert_xmu_mixed(got, ref)
         s.close()
+
+
+@pytest.mark.parametrize("fused", ["0", "1"])
+def test_mfx_pin_rules_out_the_plane_passes(tmp_path, monkeypatch, solvents, fused):
+    """R3D_MFX alone pins the per-axis passes with the mix in a kernel of its
+    own (0) or fused into the x pass (1), on grids that the plane passes take."""
+    import rism3d as R
+    import synthetic as S
+    xvk = solvents["h2o_vv"]
+    monkeypatch.setenv("R3D_MFX", fused)
+    inp = S.small(str(tmp_path), nu=6, grid=64, box=32.0, solvent=xvk)
+    s = R.RISM3D(precision="mixed")
+    s.initialize(inp, xvk=xvk)
+    s.step(3)
+    names = [k[0] for k in s.profile_kernels(2)]
+    s.close()
+    assert "fft_y_fwd" in names  # (a plane's y transform has no launch of its own)
+    assert ("mix_fx" in names) == (fused == "1") and ("mix_an2" in names) == (fused == "0")
