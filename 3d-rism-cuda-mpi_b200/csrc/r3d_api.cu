@@ -2117,6 +2117,16 @@ static int profile_typed(r3d_ctx *c, int reps, std::string &names, double *ms,
   Ctl h;
   int rc = read_ctl(c, h);
   if (rc) return rc;
+  // a forward pass that mixes is timed with its mix (r3d_step leaves none
+  // pending): request one from the last evaluation's sums
+  const bool fused = c->mixer == MIX_AN2 && (c->geo.mfx || c->geo.rt);
+  if (fused && h.step > 0 && !h.mix_flag) {
+    if (c->geo.rt)
+      launch_rt_reduce(c->ddesc, 1, 1, s);
+    else
+      launch_reduce(c->ddesc, ixc, 1, 1, s);
+    if ((rc = read_ctl(c, h))) return rc;
+  }
   const bool dots = c->mixer == MIX_AN2 && h.count_left <= 0;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
@@ -2139,7 +2149,7 @@ static int profile_typed(r3d_ctx *c, int reps, std::string &names, double *ms,
     return R3D_OK;
   };
   const double cref = d.cref ? rs : 0.0;
-  if (c->geo.mfx || (c->geo.rt && c->mixer == MIX_AN2)) {
+  if (fused) {
     // the mix fused into FX: t, u, c_ref, and (mixing) the residual and the
     // four history rows in; t, its two history entries, g and w out
     const bool mixing = h.mix_flag != 0, picard = h.coef[2] < 0;

@@ -161,6 +161,29 @@ def test_step_after_anderson_mixes_once(tmp_path, monkeypatch, solvents, prec, p
                    ("calculate", "anderson", 1, 1))
 
 
+@pytest.mark.parametrize("path,prec", [("plane_listed", "fp64"), ("plane_listed", "mixed"),
+                                       ("fused_per_axis", "mixed")])
+def test_profiled_forward_pass_mixes(tmp_path, monkeypatch, solvents, path, prec):
+    """After r3d_step nothing is pending, but the mixing forward pass is profiled
+    with its mix: bytes of t, u, (c_ref,) R and four history rows in, t, two
+    history rows, g and the spectrum out; and the next steps start from the
+    same t."""
+    import rism3d as R
+    import synthetic as S
+    grid, env = DEFERRED[path]
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    inp = S.small(str(tmp_path), nu=6, grid=grid, box=tuple(0.5 * k for k in grid), solvent=solvents["h2o_vv"])
+    s = R.RISM3D(precision=prec)
+    s.initialize(inp, xvk=solvents["h2o_vv"])
+    s.step(3)
+    t = s.get("t")
+    by = {name: b for name, _, b in s.profile_kernels(2)}
+    assert by["mix_fx"] == (96 if prec == "fp64" else 64) * 2 * np.prod(grid)
+    assert np.array_equal(s.get("t"), t)
+    s.close()
+
+
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 def test_ksave_file_holds_the_mixed_t(tmp_path, monkeypatch, solvents, prec):
     """The .tuv that iterate saves after step 3 is the t of the start of step 4."""
