@@ -1141,7 +1141,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   __shared__ double sw[M][kIntTile];                // rho_v g_v
   const int n = NS > 0 ? NS : at.n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int a = blockIdx.y * kIntAtoms + lane;
+  const int a = blockIdx.x * kIntAtoms + lane;
   const bool live = a < at.nu;
   const double ax = live ? at.x[a] : 0, ay = live ? at.y[a] : 0, az = live ? at.z[a] : 0;
   const double qa = live ? at.q[a] * at.cc : 0;
@@ -1160,7 +1160,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   double e1[M], e6[M], e12[M], en[M];          // en: energies of the near pairs
 #pragma unroll
   for (int v = 0; v < M; ++v) e1[v] = e6[v] = e12[v] = en[v] = 0;
-  const long long c0 = blockIdx.x * chunk, c1 = min(N, c0 + chunk);
+  const long long c0 = blockIdx.y * chunk, c1 = min(N, c0 + chunk);
   for (long long t0 = c0; t0 < c1; t0 += kIntTile) {
     const int nt = (int)min((long long)kIntTile, c1 - t0);
     __syncthreads();
@@ -1245,7 +1245,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       double sum = 0;
 #pragma unroll
       for (int j = 0; j < NW; ++j) sum += red[j * 32 + lane];
-      part[((long long)blockIdx.x * at.nu + a) * (4 + n) + k] = sum;
+      part[((long long)blockIdx.y * at.nu + a) * (4 + n) + k] = sum;
     }
     __syncthreads();
   }
@@ -1271,7 +1271,7 @@ void launch_atom_integrals(const IntAtoms &at, const double *g, long long N, con
                            const double *dr, double *part, int nchunk, double *out,
                            cudaStream_t s) {
   const long long chunk = (N + nchunk - 1) / nchunk;
-  dim3 gr(nchunk, (at.nu + kIntAtoms - 1) / kIntAtoms);
+  dim3 gr((at.nu + kIntAtoms - 1) / kIntAtoms, nchunk);  // (y ends at 65535: at most 1185 chunks)
 #define R3D_INT(NS)                                                                      \
   k_atom_integrals<NS><<<gr, kThreads, 0, s>>>(at, g, N, grid[0], grid[1], grid[2], dr[0], \
                                                dr[1], dr[2], chunk, part)

@@ -296,6 +296,28 @@ def test_atom_integrals_match_direct_sums(tmp_path, solvents, nu):
             assert abs(ad[a] - A * dv / kcal) <= 1e-10 * (np.abs(ad).max() + 1e-30)
 
 
+def test_atom_integrals_of_two_million_atoms(tmp_path, solvents):
+    """More groups of 32 atoms than a grid has rows (65535): the first and the
+    last atom, alike, get the same numbers; those between have no charge and no
+    depth."""
+    import rism3d as R
+    nu = 65536 * 32 + 1
+    real, ghost = "3.0 0.2 0.3 1.0 1.0 1.0\n", "3.0 0.0 0.0 0.0 0.0 0.0\n"
+    inp = str(tmp_path / "many.inp")
+    with open(inp, "w") as f:
+        f.write(" m 0 20220301\n KH\n %s\n 1.0e-6 1\n 2 0.6 0.2\n 8.0 8.0 4.0\n 16 16 8\n %d\n"
+                % (solvents["h2o_vv"], nu))
+        f.write(real + ghost * (nu - 2) + real)
+    s = R.RISM3D(precision="fp64")
+    s.initialize(inp, xvk=solvents["h2o_vv"])
+    s.iterate()
+    grad, euv, ad = s.atom_integrals()
+    s.close()
+    assert np.isfinite(grad).all() and np.abs(grad[0]).min() > 0 and np.abs(euv[0]).min() > 0
+    for a in (grad, euv, ad):
+        assert np.array_equal(a[0], a[-1]) and not a[1:-1].any()
+
+
 def test_grid_copy_to_page_locked_memory(tmp_path, solvents):
     import ctypes
     import torch
