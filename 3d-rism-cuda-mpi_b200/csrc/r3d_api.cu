@@ -674,30 +674,60 @@ static bool rt_wanted() {
   if (const char *ev = getenv("R3D_X_VARIANT")) return std::atoi(ev) == 5;
   return !getenv("R3D_AUTOTUNE") && !getenv("R3D_MFX");
 }
-// Whether the per-axis passes are the faster ones for a planned geometry: only
-// where they have compile-time-sized kernels on every axis and the plane passes
-// do not.  us per iteration, plane passes and per-axis passes:
-// - FP64 arithmetic on FP32 grids, planes in more than one round of two CTAs
-//   per SM, or tiles: four sites 80 x 72 x 96 134, 123; 64 x 72 x 80 107, 74;
-//   96 x 80 x 80 146, 123; 256 x 72 x 96 311, 222; 128 x 128 x 40 176, 110.
-//   In one round: 80 x 64 x 64 59, 79; two sites 80 x 72 x 96 56, 66.
-// - their rows of 24, 72 and 80 points (nx 48, 144, 160) are slow: four sites
-//   144 x 72 x 96 195, 236; 160 x 72 x 96 210, 224; 48 x 64 x 96 76, 80.
-// - 32^3: mixed four sites 37, 31, FP64 the same.
-// - FP64 grids, planes in more than one round, rows of 40 points or more:
-//   four sites 80 x 72 x 96 144, 137; 80 x 96 x 80 164, 153 (96 x 80 x 80 155,
-//   169); in two full rounds the plane passes: 80 x 72 x 128 164, 182.
+// Whether the per-axis passes are the faster ones for a planned geometry.  They
+// can be only where they have compile-time-sized kernels on every axis and the
+// plane passes do not: of 62 grids without such kernels on some axis (two and
+// four sites, both precisions) the plane passes took 0.12 to 0.9 of the time of
+// the per-axis ones, and 1.06 once.  Elsewhere the lines lie where 407 grids, two
+// and four sites, both precisions, changed sides (us per iteration, plane passes
+// and per-axis passes).  What decides is how much of a round of the places (two
+// CTAs per SM) the planes fill, and the rows: those of 24 and 72 points are slow
+// on the per-axis passes, those of 40 good in FP64.
+// - FP64, planes of run-time sizes: few planes leave SMs idle (two sites
+//   64 x 144 x 24 67, 47; 256 x 48 x 24 76, 49), else they win (two sites
+//   128 x 72 x 128 117, 136), but for rows of 40 with a second round under 3/4
+//   full (four sites 80 x 72 x 96 142, 137).
+// - FP64 arithmetic on FP32 grids: with rows of 72 (two sites 144 x 72 x 96 102,
+//   125), of 24 (from 89 CTAs, no second round under 0.7), and in one well-filled
+//   round with rows of 16, 40 and 48 or z kernels of listed size (four sites
+//   80 x 64 x 64 59, 77; 128 x 80 x 64 105, 117; two sites 128 x 72 x 128
+//   107, 91); not in more rounds (four sites 64 x 72 x 80 107, 74).
+// - FP32 arithmetic: but for rows of a power of two in a round under 0.6, a second
+//   under 0.8 or, up to 32, in more (two sites 64 x 160 x 80 90, 76; 256 x 64 x 192
+//   226, 196; four sites 64 x 64 x 160 137, 111; two sites 192 x 64 x 192 184, 237).
+// - Row tiles: FP64 with two axes listed (with two sites, z among them; two sites
+//   256 x 96 x 24 1.3 times); FP64 on FP32 grids with listed rows (72, or z listed
+//   too) or rows of 80 and y and z listed (160 x 144 x 144 0.87 times, 288 x 128 x 24
+//   153, 87); FP32 with four sites, z listed or listed rows of no power of two
+//   (two sites 288 x 160 x 144 398, 492; 256 x 128 x 80 191, 165).
+// - Planes of listed size with another z: but for few planes of 96^2 (two sites
+//   96 x 96 x 32, FP64, 58, 48).
+// Of these 1628 cases the rule takes the side that is over 10 % slower for 24, 21
+// of them on the per-axis passes (the worst: mixed, two sites 192 x 16 x 96 43, 60)
+// and three on the planes (mixed, four sites 48 x 40 x 192 113, 100).
 static bool per_axis_faster(const Desc &d, const Geo &g, bool fp64) {
+  if (!d.ct_x || !d.ct_y || !d.ct_z) return false;
   const int kind = fp64 ? 0 : g.rt_dbl ? 2 : 1;
-  if (kind == 1 || !d.ct_x || !d.ct_y || !d.ct_z) return false;
-  if (rt_static_x(kind, d.nx, d.ny, d.rt_plane != 0) &&
-      (d.rt_plane || rt_static_y(kind, d.ny)) && rt_static_z(kind, d.nz, d.n))
-    return false;
-  const int planes = d.n * d.nz, round = 2 * kNumSM;
-  if (fp64)
-    return d.rt_plane && d.hx >= 40 && d.hx <= 48 && planes > round && 2 * planes < 3 * round;
-  return d.hx < 24 ||
-         (d.hx >= 32 && (d.hx <= 64 || d.hx == 128) && (!d.rt_plane || planes > round));
+  const bool plane = d.rt_plane != 0, sx = rt_static_x(kind, d.nx, d.ny, plane),
+             sy = plane ? sx : rt_static_y(kind, d.ny), sz = rt_static_z(kind, d.nz, d.n);
+  if (sx && sy && sz) return false;
+  const bool pow2 = (d.hx & (d.hx - 1)) == 0;
+  if (!plane) {
+    if (kind == 2) return !((sx && (d.hx == 72 || sz)) || (d.hx == 80 && sy && sz));
+    if (kind == 0) return !(sx + sy + sz >= 2 && (d.n > 2 || sz));
+    return !(d.n > 2 || sz || (sx && !pow2));
+  }
+  const int ctas = g.rt_fctas, places = 2 * kNumSM, rounds = (ctas + places - 1) / places;
+  const double full = (double)ctas / ((double)places * rounds);
+  if (sx) return d.hx >= 48 && ctas < 96;
+  if (kind == 0) return ctas < (d.n > 2 ? 110 : 90) || (d.hx == 40 && rounds == 2 && full < 0.75);
+  if (kind == 1)
+    return pow2 && !(full >= 0.8 || (rounds == 1 && full >= 0.6) || (rounds >= 3 && d.hx > 32));
+  if (d.hx == 72) return false;
+  if (d.hx == 24) return ctas < 89 || (rounds == 2 && full < 0.7);
+  if (rounds > 1) return true;
+  if (d.hx == 16 || d.hx == 40) return ctas <= kNumSM && !(ctas >= 118 && sz);
+  return !(sz && ((d.hx == 48 && full >= 0.5) || (full >= 0.8 && full < 0.9)));
 }
 static int plan_geometry(r3d_ctx *c, Desc &d) {
   int rc = plan_geo(c, d, c->geo, c->fp64, c->prob.natv);

@@ -345,7 +345,12 @@ def test_grid_copy_to_page_locked_memory(tmp_path, solvents):
     ("mixed", 4, (64, 72, 80), False), ("mixed", 4, (80, 64, 64), True),
     ("mixed", 2, (128, 128, 40), False), ("mixed", 2, (32, 32, 32), False),
     ("mixed", 2, (48, 48, 40), True), ("fp64", 4, (80, 72, 80), False),
-    ("fp64", 4, (64, 72, 80), True)])
+    ("fp64", 4, (64, 72, 80), True),
+    # few planes; row tiles; a round that the planes fill, with other rows and z
+    ("fp64", 2, (64, 144, 24), False), ("mixed", 2, (64, 72, 48), False),
+    ("fp64", 2, (96, 96, 32), False), ("mixed", 2, (256, 128, 80), False),
+    ("mixed", 2, (288, 128, 24), False), ("mixed", 2, (128, 72, 128), False),
+    ("fp64", 4, (96, 80, 80), True), ("mixed", 4, (144, 72, 40), True)])
 def test_default_passes_by_geometry(tmp_path, monkeypatch, solvents, precision, n, dims, plane):
     import rism3d as R
     import synthetic as S
