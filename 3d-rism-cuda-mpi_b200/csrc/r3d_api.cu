@@ -40,6 +40,7 @@ size_t smem_x(int hx, int n, int S, size_t csz);
 size_t smem_y(int ny, int P, size_t csz);
 size_t smem_z(int nz, int n, int P, size_t csz);
 void kernels_set_smem(bool fp64, size_t maxbytes);
+void kernels_set_smem_for(bool fp64, size_t maxbytes, int hx, int ny, int nz);
 int dot_blocks_per_sm(bool fp64);
 int mix_chunk();
 void launch_twiddle(double2 *o64, float2 *o32, int count, double scale, cudaStream_t s);
@@ -651,6 +652,7 @@ extern "C" int r3d_set_control(r3d_ctx *c, double convergence, int maxstep) {
 static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites);
 static bool ixb_config(int device, const Desc &d, bool fp64, int pcb, Geo &g);
 static bool plan_rt(int device, Desc &d, Geo &g, bool fp64);
+static void plan_variants(r3d_ctx *c, Desc &d, Geo &g, bool fp64);
 // Whether the mixed path's plane passes compute in FP64 on its FP32 grids and
 // spectra: the transforms' roundings are by far the largest in an iteration
 // (FP32 transforms are 3e-7 of h off, the spectra's storage 4e-8), and AN2
@@ -733,10 +735,12 @@ static int plan_geometry(r3d_ctx *c, Desc &d) {
   int rc = plan_geo(c, d, c->geo, c->fp64, c->prob.natv);
   if (rc) return rc;
   c->geo.rt = rt_wanted() && plan_rt(c->opts.device, d, c->geo, c->fp64);
-  if (c->geo.rt && !getenv("R3D_X_VARIANT") && per_axis_faster(d, c->geo, c->fp64)) c->geo.rt = 0;
+  if (!c->geo.rt) plan_variants(c, d, c->geo, c->fp64);
   return R3D_OK;
 }
 
+// The passes that every geometry has (the FP64 refresh and the transform seam
+// run them, and the iteration where no variant is chosen), and the mixers.
 static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites) {
   const Problem &p = c->prob;
   d.nx = p.grid[0];
@@ -802,6 +806,25 @@ static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites) {
   g.ix_ctas = std::min(d.tiles_x, 4 * kNumSM);
   g.ix_per = (d.tiles_x + g.ix_ctas - 1) / g.ix_ctas;
   g.ix_ctas = (d.tiles_x + g.ix_per - 1) / g.ix_per;
+  // mixers: one chunk of mix_chunk() elements per CTA; ANM dots: one full
+  // wave of a grid-stride reduction
+  const long long niv = (long long)d.n * d.Ns;
+  g.mix_ctas = (int)((niv + mix_chunk() - 1) / mix_chunk());
+  int nsm = kNumSM;
+  if (c->opts.device >= 0) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->opts.device);
+  const int bps = c->opts.device >= 0 ? dot_blocks_per_sm(fp64) : 4;
+  g.dot_ctas = (int)std::min<long long>((d.N + kThreads - 1) / kThreads, (long long)nsm * bps);
+  return R3D_OK;
+}
+
+// The variants of the per-axis iteration passes that a geometry offers.  Planning
+// them opts every kernel of theirs into large shared memory and asks for
+// occupancies, which loads the kernels: a solve on the plane passes skips it
+// (r3d_initialize of a process' first solve, 96^3 mixed: 230 to 255 ms against
+// 290 to 350, 64^3 FP64 130 against 160).
+static void plan_variants(r3d_ctx *c, Desc &d, Geo &g, bool fp64) {
+  const size_t cs = fp64 ? 16 : 8;
+  const int rowsN = d.ny * d.nz;
   g.ixb_pc = 0;
   if (d.ct_x) {  // bulk-staged IX: as many CTAs as stay resident
     const int pcb = fp64 ? 4 : 8;
@@ -952,15 +975,6 @@ static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites) {
       g.zp_ctas = occ * nsm;
     }
   }
-  // mixers: one chunk of mix_chunk() elements per CTA; ANM dots: one full
-  // wave of a grid-stride reduction
-  const long long niv = (long long)d.n * d.Ns;
-  g.mix_ctas = (int)((niv + mix_chunk() - 1) / mix_chunk());
-  int nsm = kNumSM;
-  if (c->opts.device >= 0) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->opts.device);
-  const int bps = c->opts.device >= 0 ? dot_blocks_per_sm(fp64) : 4;
-  g.dot_ctas = (int)std::min<long long>((d.N + kThreads - 1) / kThreads, (long long)nsm * bps);
-  return R3D_OK;
 }
 
 // ------------------------------------------------------------ plane passes
@@ -978,7 +992,7 @@ static int rt_index_at(const RtPlan &p, int P) {
 
 // Launch geometry of the plane passes; false where they do not cover the
 // grid (a length with a prime factor over 13, more than four sites, an odd
-// nz).
+// nz) or the per-axis passes are faster.
 static bool plan_rt(int device, Desc &d, Geo &g, bool fp64) {
   g.rt_dbl = !fp64 && rt_double(d);
   const int kind = fp64 ? 0 : g.rt_dbl ? 2 : 1;
@@ -1013,6 +1027,8 @@ static bool plan_rt(int device, Desc &d, Geo &g, bool fp64) {
   g.rt_smy = rt_smem_y(d.ny, d.rt_pcy, cs);
   g.rt_smz = rt_smem_z(d.nz, d.n, pcz, cs);
   if (g.rt_smx > kSmemMax || g.rt_smy > kSmemMax || g.rt_smz > kSmemMax) return false;
+  g.rt_fctas = d.n * d.rt_tps;
+  if (!getenv("R3D_X_VARIANT") && per_axis_faster(d, g, fp64)) return false;
   g.rt_nt = rt_threads(d, kind, kNumSM);
   int occ = 0;
   if (fp64) {
@@ -1036,7 +1052,6 @@ static bool plan_rt(int device, Desc &d, Geo &g, bool fp64) {
     d.rt_iper = (d.rt_tps + want - 1) / want;
     d.rt_icps = (d.rt_tps + d.rt_iper - 1) / d.rt_iper;
   }
-  g.rt_fctas = d.n * d.rt_tps;
   g.rt_ictas = d.n * d.rt_icps;
   g.rt_yctas = d.rt_plane ? 0 : d.n * d.nz * ((d.hx + d.rt_pcy - 1) / d.rt_pcy);
   g.rt_zctas = d.ny * ((d.hx + pcz - 1) / pcz);
@@ -1413,7 +1428,7 @@ static int refresh(r3d_ctx *c, bool zero) {
   CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), s));
   CK(copy_h2d(c, dd, &dr, sizeof(Desc), s));
   CK(copy_h2d(c, pre, pf, sizeof(pf), s));
-  kernels_set_smem(true, kSmemMax);
+  kernels_set_smem_for(true, kSmemMax, d.hx, d.ny, d.nz);
   pass_fx<P64>(dr, g, Batch{dd, pre, 1}, s, 0, c64);
   pass_fy<P64>(dr, g, Batch{dd, pre + 2, 1}, s, -1, 0);
   pass_zoz<P64>(dr, g, Batch{dd, pre + 4, 1}, s, 2, 0);
@@ -1884,8 +1899,8 @@ static int init_typed(r3d_ctx *c, const ShellTable &st) {
   }
   // the attribute is a per-function limit shared by every context: always
   // allow the largest tile any context may choose (set before any capture)
-  kernels_set_smem(c->fp64, kSmemMax);
-  kernels_set_smem(true, kSmemMax);
+  if (!c->fp64 && !c->geo.rt) kernels_set_smem_for(false, kSmemMax, d.hx, d.ny, d.nz);
+  kernels_set_smem_for(true, kSmemMax, d.hx, d.ny, d.nz);
   CK(cudaGetLastError());
   return R3D_OK;
 }
@@ -2904,7 +2919,7 @@ static int fft_typed(r3d_ctx *c, int nx, int ny, int nz, const double *box, int 
   const int *dp = (const int *)pre;
   Batch bx{(Desc *)ddesc, dp, 1}, by{(Desc *)ddesc, dp + 2, 1}, bz{(Desc *)ddesc, dp + 4, 1},
       bix{(Desc *)ddesc, dp + 6, 1};
-  kernels_set_smem(c->fp64, kSmemMax);
+  kernels_set_smem_for(c->fp64, kSmemMax, d.hx, d.ny, d.nz);
   const double dv = box[0] * box[1] * box[2] / (double)N;
   const int par0 = ((nx + ny + nz) / 2) & 1;
   std::vector<double> tmp(std::max(N, 2 * Nh));
@@ -2968,7 +2983,7 @@ extern "C" int r3d_fft3d(int device, int precision, int nx, int ny, int nz,
     return fail(nullptr, R3D_EINVAL, "fft3d: nx must be even >= 4");
   }
   Desc d{};
-  rc = plan_geometry(c, d);
+  rc = plan_geo(c, d, c->geo, c->fp64, 1);
   if (!rc) {
     c->desc = d;
     rc = c->fp64 ? fft_typed<P64>(c, nx, ny, nz, box, dir, in, out)

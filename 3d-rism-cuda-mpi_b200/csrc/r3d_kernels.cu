@@ -1641,6 +1641,8 @@ void launch_twiddle(double2 *o64, float2 *o32, int count, double scale, cudaStre
 
 template <typename P>
 void ct_allow_smem_all();
+template <typename P>
+void ct_allow_smem_for(int hx, int ny, int nz);
 
 template <typename P>
 void tma_allow_smem_all();
@@ -1659,6 +1661,19 @@ void kernels_set_smem(bool fp64, size_t maxbytes) {
       tma_allow_smem_all<PMix>();
     }
     ct_done[fp64] = true;
+  }
+}
+
+// The same for one geometry: the general kernels and the compile-time-sized
+// ones of its lengths (opting a kernel in loads it: 270 of them took a quarter
+// of a second of a process' first solve).
+void kernels_set_smem_for(bool fp64, size_t maxbytes, int hx, int ny, int nz) {
+  if (fp64) {
+    set_smem_attrs<P64>(maxbytes);
+    ct_allow_smem_for<P64>(hx, ny, nz);
+  } else {
+    set_smem_attrs<PMix>(maxbytes);
+    ct_allow_smem_for<PMix>(hx, ny, nz);
   }
 }
 

@@ -1408,6 +1408,31 @@ void ct_allow_smem_all() {
   allow_smem(k_ix_warp<P, 512, 2>);
 }
 template void ct_allow_smem_all<PCT>();
+// The tile-per-CTA kernels of one geometry (half rows of hx points).
+template <typename P>
+void ct_allow_smem_for(int hx, int ny, int nz) {
+  constexpr int PX = sizeof(typename P::R) == 4 ? 32 : 16;
+#define R3D_ATTR(LL)                         \
+  if (hx == LL) {                            \
+    allow_smem(k_fx_ct<P, LL, PX, 0>);       \
+    allow_smem(k_fx_ct<P, LL, PX, 1>);       \
+    allow_smem(k_ix_ct<P, LL, PX, 0>);       \
+    allow_smem(k_ix_ct<P, LL, PX, 1>);       \
+  }                                          \
+  if (ny == LL) {                            \
+    allow_smem(k_fy_ct<P, LL, 8, -1>);       \
+    allow_smem(k_fy_ct<P, LL, 8, 1>);        \
+    allow_smem(k_fy_ct<P, LL, 16, -1>);      \
+    allow_smem(k_fy_ct<P, LL, 16, 1>);       \
+  }                                          \
+  if (nz == LL) {                            \
+    allow_smem(k_zoz_ct<P, LL, 4>);          \
+    allow_smem(k_zoz_ct<P, LL, 8>);          \
+  }
+  R3D_CT_LENGTHS(R3D_ATTR)
+#undef R3D_ATTR
+}
+template void ct_allow_smem_for<PCT>(int, int, int);
 
 template bool ct_launch_fx<PCT>(int, int, Batch, int, size_t, cudaStream_t, int, const void *);
 template bool ct_launch_fy<PCT>(int, int, Batch, int, size_t, cudaStream_t, int, int);
