@@ -39,8 +39,8 @@ struct AtomTab {
 size_t smem_x(int hx, int n, int S, size_t csz);
 size_t smem_y(int ny, int P, size_t csz);
 size_t smem_z(int nz, int n, int P, size_t csz);
-void kernels_set_smem(bool fp64, size_t maxbytes);
 void kernels_set_smem_for(bool fp64, size_t maxbytes, int hx, int ny, int nz);
+void kernels_set_smem_variants(bool fp64, int hx, int ny, int nz);
 int dot_blocks_per_sm(bool fp64);
 int mix_chunk();
 void launch_twiddle(double2 *o64, float2 *o32, int count, double scale, cudaStream_t s);
@@ -204,7 +204,7 @@ constexpr size_t kRtPlaneMax = 92 * 1024;
 inline int bulk_per_sm(int device, bool fp64, int which, int L, int PC, size_t smem) {
   int nb = 0;
   if (device >= 0) {
-    kernels_set_smem(fp64, kSmemMax);  // the occupancy query honours the opt-in limit
+    kernels_set_smem_variants(fp64, L, 0, 0);  // the occupancy query honours the opt-in limit
     if (which < 2)
       nb = fp64 ? ct_occupancy_bulk<P64>(which, L, PC, smem)
                 : ct_occupancy_bulk<PMix>(which, L, PC, smem);
@@ -820,8 +820,9 @@ static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites) {
 // The variants of the per-axis iteration passes that a geometry offers.  Planning
 // them opts every kernel of theirs into large shared memory and asks for
 // occupancies, which loads the kernels: a solve on the plane passes skips it
-// (r3d_initialize of a process' first solve, 96^3 mixed: 230 to 255 ms against
-// 290 to 350, 64^3 FP64 130 against 160).
+// (r3d_initialize of a process' first solve, this and opt-ins by length alone:
+// 96^3 mixed 110 ms against 300, 64^3 FP64 110 against 160, 144^3 mixed 128 against
+// 310).
 static void plan_variants(r3d_ctx *c, Desc &d, Geo &g, bool fp64) {
   const size_t cs = fp64 ? 16 : 8;
   const int rowsN = d.ny * d.nz;
@@ -890,7 +891,7 @@ static void plan_variants(r3d_ctx *c, Desc &d, Geo &g, bool fp64) {
       g.smfyt = ny_st * sby;
       g.smzt = nz_st * sbz;
       const int ty = d.n * d.nz * (d.hx / py), tz = d.ny * (d.hx / pz);
-      kernels_set_smem(fp64, kSmemMax);
+      kernels_set_smem_variants(fp64, 0, d.ny, d.nz);
       int oy = fp64 ? tma_occupancy<P64>(0, d.ny, g.smfyt) : tma_occupancy<PMix>(0, d.ny, g.smfyt);
       int oz = fp64 ? tma_occupancy<P64>(1, d.nz, g.smzt) : tma_occupancy<PMix>(1, d.nz, g.smzt);
       if (oy <= 0 || oz <= 0) g.yz_tma = 0;  // no kernels for these lengths
@@ -909,7 +910,7 @@ static void plan_variants(r3d_ctx *c, Desc &d, Geo &g, bool fp64) {
     const int pc = ct_mfx_pc(d.hx);
     const size_t sm = ct_smem_mfx(d.hx, pc);
     if (rowsN % pc == 0 && d.ny >= pc && sm <= kSmemMax) {  // rows wrap z once at most
-      kernels_set_smem(false, kSmemMax);
+      kernels_set_smem_variants(false, d.hx, 0, 0);
       const int per_sm = ct_occupancy_mfx<PMix>(d.hx, sm);
       if (per_sm > 0) {
         const int tiles = d.n * (rowsN / pc);

@@ -1640,40 +1640,36 @@ void launch_twiddle(double2 *o64, float2 *o32, int count, double scale, cudaStre
 }
 
 template <typename P>
-void ct_allow_smem_all();
-template <typename P>
 void ct_allow_smem_for(int hx, int ny, int nz);
-
 template <typename P>
-void tma_allow_smem_all();
+void ct_allow_variants(int hx);
+template <typename P>
+void tma_allow_smem(int ny, int nz);
+
+// Opt-ins into large shared memory; each loads its kernel, and with the first
+// kernel of an object the object's code, so a solve asks only for its own: the
+// general kernels; with hx (half rows), ny and nz the tile-per-CTA ones of
+// these lengths; and the staged variants of the iteration's passes.
 void kernels_set_smem(bool fp64, size_t maxbytes) {
-  static bool ct_done[2] = {false, false};
   if (fp64)
     set_smem_attrs<P64>(maxbytes);
   else
     set_smem_attrs<PMix>(maxbytes);
-  if (!ct_done[fp64]) {  // compile-time-engine passes, once per process
-    if (fp64) {
-      ct_allow_smem_all<P64>();
-      tma_allow_smem_all<P64>();
-    } else {
-      ct_allow_smem_all<PMix>();
-      tma_allow_smem_all<PMix>();
-    }
-    ct_done[fp64] = true;
-  }
 }
-
-// The same for one geometry: the general kernels and the compile-time-sized
-// ones of its lengths (opting a kernel in loads it: 270 of them took a quarter
-// of a second of a process' first solve).
 void kernels_set_smem_for(bool fp64, size_t maxbytes, int hx, int ny, int nz) {
-  if (fp64) {
-    set_smem_attrs<P64>(maxbytes);
+  kernels_set_smem(fp64, maxbytes);
+  if (fp64)
     ct_allow_smem_for<P64>(hx, ny, nz);
-  } else {
-    set_smem_attrs<PMix>(maxbytes);
+  else
     ct_allow_smem_for<PMix>(hx, ny, nz);
+}
+void kernels_set_smem_variants(bool fp64, int hx, int ny, int nz) {
+  if (fp64) {
+    ct_allow_variants<P64>(hx);
+    tma_allow_smem<P64>(ny, nz);
+  } else {
+    ct_allow_variants<PMix>(hx);
+    tma_allow_smem<PMix>(ny, nz);
   }
 }
 

@@ -1,6 +1,9 @@
 // r3d_passes_ct.cu -- the five grid passes on the compile-time FFT engine
 // (r3d_fft_ct.cuh).  Compiled once per precision: R3D_CT_FP64 = 1 builds the
-// FP64 instantiations, 0 the mixed-precision ones.  The passes compute the
+// FP64 instantiations, 0 the mixed-precision ones; and in two parts, so that a
+// solve loads the one it runs: R3D_CT_PART = 0 the tile-per-CTA passes (which the
+// FP64 refresh and the transform seam run too), 1 the iteration's staged, warp-tile
+// and mix-fused variants.  The passes compute the
 // same quantities as the runtime-length passes in r3d_kernels.cu (which stay
 // as the fallback for lengths outside kCtLengths); see that file for the
 // algorithm and the reference lines each step follows.
@@ -10,6 +13,9 @@
 
 #ifndef R3D_CT_FP64
 #define R3D_CT_FP64 1
+#endif
+#ifndef R3D_CT_PART
+#define R3D_CT_PART 0
 #endif
 
 namespace r3d {
@@ -437,7 +443,7 @@ struct IxStage {  // byte layout of one stage of staged inputs
   static constexpr size_t w = r1 + (size_t)PC * NX * sizeof(typename P::R);  // spectrum rows
   static constexpr size_t bytes = w + (size_t)PC * L * 2 * sizeof(typename P::R);
 };
-#if R3D_CT_FP64
+#if R3D_CT_FP64 && R3D_CT_PART == 0
 size_t ct_smem_ixb(int L, int PC, size_t csz, size_t rsz, size_t tsz) {
   const size_t buf = ((csz * (size_t)L * (PC + 1) + 127) / 128) * 128;
   const size_t stage = (size_t)PC * 2 * L * (tsz + 3 * rsz) + (size_t)PC * L * csz;
@@ -614,7 +620,7 @@ struct FxStage {
   static constexpr size_t cref = u + (size_t)PC * NX * sizeof(typename P::R);
   static constexpr size_t bytes = cref + (size_t)PC * NX * sizeof(typename P::R);
 };
-#if R3D_CT_FP64
+#if R3D_CT_FP64 && R3D_CT_PART == 0
 size_t ct_smem_fxb(int L, int PC, size_t csz, size_t rsz, size_t tsz) {
   const size_t buf = ((csz * (size_t)L * (PC + 1) + 127) / 128) * 128;
   return buf + 2 * (size_t)PC * 2 * L * (tsz + 2 * rsz);
@@ -751,7 +757,7 @@ struct MfxStage {
   static constexpr size_t r1 = r0 + (size_t)PC * NX * 4;
   static constexpr size_t bytes = r1 + (size_t)PC * NX * 4;
 };
-#if R3D_CT_FP64
+#if R3D_CT_FP64 && R3D_CT_PART == 0
 size_t ct_smem_mfx(int L, int PC) {
   const size_t buf = ((8 * (size_t)L * (PC + 1) + 127) / 128) * 128;
   return buf + 2 * (size_t)PC * 2 * L * (8 + 7 * 4);
@@ -924,7 +930,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 // persistent; the warps of a solve's CTAs stride over its tiles.
 constexpr int kWarps = kThreads / 32;
 
-#if R3D_CT_FP64
+#if R3D_CT_FP64 && R3D_CT_PART == 0
 size_t ct_smem_warp(int L, int PCW, size_t csz) {
   return (size_t)kWarps * L * (PCW + 1) * csz;
 }
@@ -1102,7 +1108,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(typename P::R) == 4 ? 3 : 2)
 // ------------------------------------------------------------ launchers
 #define R3D_CT_LENGTHS(X) X(16) X(24) X(32) X(40) X(48) X(64) X(72) X(80) X(96) X(128) X(144) X(160) X(192) X(256) X(512)
 
-#if R3D_CT_FP64
+#if R3D_CT_FP64 && R3D_CT_PART == 0
 size_t ct_smem_x(int L, int PC, size_t csz) { return csz * (size_t)L * (PC + 1); }
 size_t ct_smem_y(int L, int PC, size_t csz) { return csz * (size_t)L * PC; }
 size_t ct_smem_z(int L, int PC, int n, size_t csz) { return csz * (size_t)L * PC * n; }
@@ -1114,9 +1120,8 @@ bool ct_length_ok(int L) {
 }
 #endif
 
-// Every instantiation is opted into large dynamic shared memory by
-// ct_allow_smem (called at context setup: the attribute cannot be set while a
-// stream is being captured into a graph).
+// Opt-in into large dynamic shared memory, at context setup: the attribute
+// cannot be set while a stream is being captured into a graph.
 template <typename K>
 static void allow_smem(K kern) {
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
@@ -1283,7 +1288,7 @@ int ct_occupancy_mfx(int L, size_t smem) {
 #endif
   return nb;
 }
-#if R3D_CT_FP64
+#if R3D_CT_FP64 && R3D_CT_PART == 0
 int ct_mfx_pc(int L) { return mfx_pc(L); }
 #endif
 
@@ -1369,45 +1374,37 @@ int ct_occupancy_xw(int which, int L, int PCW, size_t smem) {
   return 0;
 }
 
+// The variants of the x passes for half rows of hx points.
 template <typename P>
-void ct_allow_smem_all() {
-  using R = typename P::R;
-  constexpr int PX = sizeof(R) == 4 ? 32 : 16;
-#define R3D_ATTR(LL)                                                      \
-  allow_smem(k_fx_ct<P, LL, PX, 0>);                                      \
-  allow_smem(k_fx_ct<P, LL, PX, 1>);                                      \
-  allow_smem(k_ix_ct<P, LL, PX, 0>);                                      \
-  allow_smem(k_ix_ct<P, LL, PX, 1>);                                      \
-  allow_smem(k_fy_ct<P, LL, 8, -1>);                                      \
-  allow_smem(k_fy_ct<P, LL, 8, 1>);                                       \
-  allow_smem(k_fy_ct<P, LL, 16, -1>);                                     \
-  allow_smem(k_fy_ct<P, LL, 16, 1>);                                      \
-  allow_smem(k_zoz_ct<P, LL, 4>);                                         \
-  allow_smem(k_zoz_ct<P, LL, 8>);                                         \
-  allow_smem(k_ix_bulk<P, LL, (sizeof(typename P::R) == 4 ? 8 : 4)>);      \
-  allow_smem(k_ix_bulk<P, LL, (sizeof(typename P::R) == 4 ? 4 : 2)>);      \
-  allow_smem(k_fx_bulk<P, LL, (sizeof(typename P::R) == 4 ? 8 : 4)>);       \
-  allow_smem(k_fx_warp<P, LL, 4>);                                        \
-  allow_smem(k_ix_warp<P, LL, 4>);
+void ct_allow_variants(int hx) {
+  constexpr int PB = sizeof(typename P::R) == 4 ? 8 : 4;
+#define R3D_ATTR(LL)                      \
+  if (hx == LL) {                         \
+    allow_smem(k_ix_bulk<P, LL, PB>);     \
+    allow_smem(k_ix_bulk<P, LL, PB / 2>); \
+    allow_smem(k_fx_bulk<P, LL, PB>);     \
+    allow_smem(k_fx_warp<P, LL, 4>);      \
+    allow_smem(k_ix_warp<P, LL, 4>);      \
+  }
   R3D_CT_LENGTHS(R3D_ATTR)
 #undef R3D_ATTR
-  allow_smem(k_fx_bulk<P, 256, (sizeof(typename P::R) == 4 ? 4 : 2)>);
-  allow_smem(k_fx_bulk<P, 512, (sizeof(typename P::R) == 4 ? 4 : 2)>);
-  if constexpr (sizeof(typename P::R) == 4) {
-    allow_smem(k_ix_bulk<P, 256, 2>);
-    allow_smem(k_ix_bulk<P, 512, 2>);
+#define R3D_ATTR(LL)                                                          \
+  if (hx == LL) {                                                             \
+    allow_smem(k_fx_bulk<P, LL, PB / 2>);                                     \
+    if constexpr (sizeof(typename P::R) == 4) allow_smem(k_ix_bulk<P, LL, 2>); \
+    allow_smem(k_fx_warp<P, LL, 2>);                                          \
+    allow_smem(k_ix_warp<P, LL, 2>);                                          \
   }
-  allow_smem(k_fx_warp<P, 256, 2>);
-  allow_smem(k_fx_warp<P, 512, 2>);
+  R3D_ATTR(256)
+  R3D_ATTR(512)
+#undef R3D_ATTR
 #if !R3D_CT_FP64
-#define R3D_AMFX(LL) allow_smem(k_mfx_bulk<LL, mfx_pc(LL)>);
-  R3D_CT_LENGTHS(R3D_AMFX)
-#undef R3D_AMFX
+#define R3D_ATTR(LL) \
+  if (hx == LL) allow_smem(k_mfx_bulk<LL, mfx_pc(LL)>);
+  R3D_CT_LENGTHS(R3D_ATTR)
+#undef R3D_ATTR
 #endif
-  allow_smem(k_ix_warp<P, 256, 2>);
-  allow_smem(k_ix_warp<P, 512, 2>);
 }
-template void ct_allow_smem_all<PCT>();
 // The tile-per-CTA kernels of one geometry (half rows of hx points).
 template <typename P>
 void ct_allow_smem_for(int hx, int ny, int nz) {
@@ -1432,12 +1429,14 @@ void ct_allow_smem_for(int hx, int ny, int nz) {
   R3D_CT_LENGTHS(R3D_ATTR)
 #undef R3D_ATTR
 }
+#if R3D_CT_PART == 0
 template void ct_allow_smem_for<PCT>(int, int, int);
-
 template bool ct_launch_fx<PCT>(int, int, Batch, int, size_t, cudaStream_t, int, const void *);
 template bool ct_launch_fy<PCT>(int, int, Batch, int, size_t, cudaStream_t, int, int);
 template bool ct_launch_zoz<PCT>(int, int, Batch, int, size_t, cudaStream_t, int);
 template bool ct_launch_ix<PCT>(int, int, Batch, int, size_t, cudaStream_t, int, void *, int);
+#else
+template void ct_allow_variants<PCT>(int);
 template bool ct_launch_ixb<PCT>(int, int, Batch, int, size_t, cudaStream_t, int);
 template bool ct_launch_fxb<PCT>(int, int, Batch, int, size_t, cudaStream_t, int);
 template bool ct_launch_mfx<PCT>(int, Batch, int, size_t, cudaStream_t, int, int);
@@ -1445,5 +1444,6 @@ template int ct_occupancy_mfx<PCT>(int, size_t);
 template int ct_occupancy_bulk<PCT>(int, int, int, size_t);
 template bool ct_launch_xw<PCT>(int, int, int, Batch, int, size_t, cudaStream_t);
 template int ct_occupancy_xw<PCT>(int, int, int, size_t);
+#endif
 
 }  // namespace r3d

@@ -368,16 +368,19 @@ int tma_occupancy(int which, int L, size_t smem) {
   return 0;
 }
 
+// opt-in into large dynamic shared memory: columns of ny and of nz points
 template <typename P>
-void tma_allow_smem_all() {
+void tma_allow_smem(int ny, int nz) {
   constexpr int PY = tma_pc_y<P>(), PZ = tma_pc_z<P>();
   auto allow = [](const void *f) {
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
   };
-#define R3D_TATTR(LL)                                  \
-  allow((const void *)k_fy_tma<P, LL, PY, -1>);        \
-  allow((const void *)k_fy_tma<P, LL, PY, 1>);         \
-  allow((const void *)k_zoz_tma<P, LL, PZ>);
+#define R3D_TATTR(LL)                             \
+  if (ny == LL) {                                 \
+    allow((const void *)k_fy_tma<P, LL, PY, -1>); \
+    allow((const void *)k_fy_tma<P, LL, PY, 1>);  \
+  }                                               \
+  if (nz == LL) allow((const void *)k_zoz_tma<P, LL, PZ>);
   R3D_TMA_LENGTHS(R3D_TATTR)
 #undef R3D_TATTR
 }
@@ -385,6 +388,6 @@ void tma_allow_smem_all() {
 template bool tma_launch_fy<PTM>(int, int, Batch, int, size_t, cudaStream_t, int, int);
 template bool tma_launch_zoz<PTM>(int, Batch, int, size_t, cudaStream_t, int, int);
 template int tma_occupancy<PTM>(int, int, size_t);
-template void tma_allow_smem_all<PTM>();
+template void tma_allow_smem<PTM>(int, int);
 
 }  // namespace r3d
