@@ -8,8 +8,11 @@ integrals for atom counts around a warp, and grid copies to page-locked memory.
 
 Tolerances: three evaluations and mixes in FP64 differ by roundings of order
 1e-15, and each mix multiplies a difference of R by less than 30 at contact
-peaks: 1e-10 of t's largest value.  The mixed path's transforms round to about
-3e-7 of c: 1e-4 of t's largest value after the same three steps."""
+peaks: 1e-10 of t's largest value.  In mixed precision the general passes'
+transforms, and those of the plane passes in FP32 arithmetic, round to about
+3e-7 of c: 1e-4 of t's largest value after the same three steps.  The plane
+passes in FP64 arithmetic on FP32 grids (most grids below 3.5 million voxels)
+are also held to the FP64 solve, see test_fp64_arithmetic_on_fp32_grids."""
 import gzip
 import os
 
@@ -56,6 +59,14 @@ def _three_steps(R, inp, xvk, prec):
     ((256, 10, 18), 4),     # row tiles, the last of them partial
     ((200, 126, 12), 2),    # run-time sizes, 7 x 18 columns
     ((8, 6, 4), 2),         # the smallest
+    # mixed: FP32 arithmetic (lengths all listed, an FP64 plan of a pass more)
+    ((48, 48, 128), 2),     # a run-time plane, a compile-time z of radices 16 and 8
+    ((128, 128, 32), 2),    # mixed: FP64 arithmetic in tiles (32 is not listed)
+    ((128, 128, 128), 1),   # compile-time planes
+    # and above 3.5 million voxels: run-time tiles, several per inverse CTA, the
+    # last partial; odd half rows of 7 x 11 and 7 x 13
+    ((154, 150, 156), 2),
+    ((182, 144, 150), 1),
 ])
 def test_plane_passes_match_general_passes(tmp_path, monkeypatch, grid, sites, prec):
     import rism3d as R
@@ -100,6 +111,24 @@ def test_fp64_step_leaves_the_mixed_t(tmp_path, monkeypatch, solvents, n):
         d = np.abs(out["5"][k] - out["0"][k]).max()
         assert d <= 1e-10 * np.abs(out["0"][k]).max()
     assert out["5"][2] == out["0"][2] == n + 2
+
+
+@pytest.mark.parametrize("grid,sites", [((48, 48, 48), 2), ((90, 22, 26), 3), ((44, 52, 28), 1),
+                                        ((200, 126, 12), 2), ((96, 32, 36), 4)])
+def test_fp64_arithmetic_on_fp32_grids(tmp_path, monkeypatch, grid, sites):
+    """Three mixed steps against three FP64 ones on the plane passes.  What the
+    mixed path stores in FP32: u, up to 4 where g is large (half an ulp, 1.2e-7,
+    times g < 30: 4e-6 of g) and R and the long-range term, up to 30 (1e-6); the
+    spectra's roundings average out in the transforms.  5e-6 per evaluation:
+    2e-5 of t's largest value after three."""
+    import rism3d as R
+    import synthetic as S
+    xvk = _subset_xvk(str(tmp_path / "s.xvk"), sites)
+    sol = S.make_solute(4, 3, radius=0.9, dmin=0.5, sig=(2.5, 3.0), qsd=0.2)
+    inp = S.write_inp(str(tmp_path / "p.inp"), sol, tuple(0.5 * n for n in grid), grid, xvk)
+    monkeypatch.setenv("R3D_X_VARIANT", "5")
+    t = {p: _three_steps(R, inp, xvk, p)[1] for p in ("fp64", "mixed")}
+    assert np.abs(t["mixed"] - t["fp64"]).max() <= 2e-5 * np.abs(t["fp64"]).max()
 
 
 # the paths whose next forward pass mixes (a listed and an unlisted row length
