@@ -29,13 +29,17 @@ def _make(R, refcase, deck, over, prec):
     return s
 
 
-@pytest.mark.parametrize("passes", ["table", "persistent_z"])
+@pytest.mark.parametrize("passes", ["default", "per_axis", "persistent_z"])
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 def test_batch_equals_solo(refcase, tmp_path, monkeypatch, prec, passes):
-    """passes: the committed variant table, or the Stockham x passes with the
-    persistent z pass (one CTA per SM walking the tiles of every solve of a
-    launch, skipping those of finished solves)."""
+    """passes: those that the geometries' rule takes; the per-axis passes as they
+    run where the rule takes them (staged x passes, mixed with the mix fused into
+    the first); or the Stockham x passes with the persistent z pass (one CTA per
+    SM walking the tiles of every solve of a launch, skipping those of finished
+    solves)."""
     import rism3d as R
+    if passes == "per_axis":
+        monkeypatch.setenv("R3D_MFX", "1")
     if passes == "persistent_z":
         monkeypatch.setenv("R3D_X_VARIANT", "4")
         monkeypatch.setenv("R3D_YZ_VARIANT", "5")

@@ -10,7 +10,7 @@ RMS ends the solve as diverged).
 - A NaN planted in the initial t on the host, uploaded through r3d_set_t,
   ends that solve as DIVERGED at its first evaluation, alone and inside a
   batch, where its mates end byte for byte where they end alone.
-- The same solve run twice (fresh contexts, the committed variant table)
+- The same solve run twice (fresh contexts, the passes that the rule takes)
   gives the same step count and bitwise-identical g and .xmu, in both
   precisions."""
 import numpy as np
@@ -90,7 +90,7 @@ def test_nan_in_initial_t_diverges_alone_and_in_a_batch(refcase, tmp_path, prec)
 @pytest.mark.parametrize("prec", ["fp64", "mixed"])
 @pytest.mark.parametrize("case", ["s64nacl", "test1"])
 def test_same_solve_twice_is_bitwise_identical(refcase, tmp_path, prec, case):
-    """The pass variants come from the committed table, not from timings taken
+    """The passes come from fixed rules on the geometry, not from timings taken
     at run time, so two runs of a deck agree to the last bit."""
     import rism3d as R
     inp, xvk = refcase(case)

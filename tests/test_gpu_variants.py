@@ -1,7 +1,7 @@
-"""Every implementation of the iteration's x passes (one tile per CTA,
+"""Every implementation of the per-axis iteration's x passes (one tile per CTA,
 bulk-copy staged, warp tiles, bulk-copy staged with half-size tiles, the
-register-pass Stockham engine; a committed table picks one per geometry) and
-of its y/z passes solves to the
+register-pass Stockham engine; a rule picks one per geometry that the plane
+passes do not take) and of its y/z passes solves to the
 reference's results (or the oracle's, for grids the reference cannot run):
 same steps (within 1), .xmu within 1e-6 kcal/mol."""
 import os
