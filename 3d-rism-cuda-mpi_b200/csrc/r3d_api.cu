@@ -992,8 +992,8 @@ static int rt_index_at(const RtPlan &p, int P) {
 }
 
 // Launch geometry of the plane passes; false where they do not cover the
-// grid (a length with a prime factor over 13, more than four sites, an odd
-// nz) or the per-axis passes are faster.
+// grid (a length that takes five passes, more than four sites; an odd nz, which
+// the deck reader refuses) or the per-axis passes are faster.
 static bool plan_rt(int device, Desc &d, Geo &g, bool fp64) {
   g.rt_dbl = !fp64 && rt_double(d);
   const int kind = fp64 ? 0 : g.rt_dbl ? 2 : 1;

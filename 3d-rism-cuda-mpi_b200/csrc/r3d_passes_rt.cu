@@ -23,6 +23,10 @@
 // in vectors (every load of a thread's voxels issued before the first use),
 // not through shared-memory staging: the tile then leaves room for more CTAs
 // per SM, whose phases (loads, transforms, stores) overlap.
+//
+// Debug builds check the indexes of the real grids, the spectrum, the shell index
+// and the partials (R3D_IN); the position tables are indexed by a tile's own
+// positions, the chi table of a non-cubic cell by the shell index as it is stored.
 #include "r3d_common.cuh"
 #include "r3d_fft_rt.cuh"
 #include "r3d_reduce.cuh"
@@ -35,6 +39,9 @@
 #ifndef R3D_RT_PART
 #define R3D_RT_PART 0
 #endif
+
+// element i of the kernel's part of the spectrum (w), checked in debug builds
+#define R3D_W(i) R3D_IN(d, w - (const S *)d.w + (i), d.n * d.Nhs)
 
 namespace r3d {
 
@@ -319,7 +326,7 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_fwd(Batch b, int allow_mix) {
   if (!plane) {
     for (int e = threadIdx.x; e < nrow * hx; e += NT) {
       const int r = rt_div(e, mghx), p = e - r * hx;
-      w[e] = rt_cvt<S>(buf[r * LDX + p]);
+      if (R3D_W(e)) w[e] = rt_cvt<S>(buf[r * LDX + p]);
     }
     return;
   }
@@ -330,7 +337,9 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_fwd(Batch b, int allow_mix) {
     rt_edge<NY, RM>(
         NY ? 0 : d.rty.n, s,
         [&] {
-          auto st = [&](int p, int y, C a) { w[y * hx + p] = rt_cvt<S>(a); };
+          auto st = [&](int p, int y, C a) {
+            if (R3D_W(y * hx + p)) w[y * hx + p] = rt_cvt<S>(a);
+          };
           rt_pass_s<NY, -1, NT, RM>(d.rty, s, hx, mghx, twy, ld, st);
         },
         [&] {
@@ -369,12 +378,12 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_y(Batch b) {
     const bool last = (int)s == (DIR < 0 ? (NY ? rt_plan_of(NY, RM).n : n) - 1 : 0);
     auto ld = [&](int p, int y) {
       if (!first) return buf[y * PC + p];
-      return p < pc ? rt_cvt<C>(w[y * hx + p]) : C{0, 0};
+      return p < pc && R3D_W(y * hx + p) ? rt_cvt<C>(w[y * hx + p]) : C{0, 0};
     };
     auto st = [&](int p, int y, C a) {
       if (!last)
         buf[y * PC + p] = a;
-      else if (p < pc)
+      else if (p < pc && R3D_W(y * hx + p))
         w[y * hx + p] = rt_cvt<S>(a);
     };
     rt_pass_s<NY, DIR, NT, RM>(d.rty, s, PC, mg, tw, ld, st);
@@ -418,7 +427,7 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_zoz(Batch b) {
     auto ld = [&](int c, int z) {
       if (!first) return lds(c, z);
       const int p = c % PC, v = c / PC;
-      return p < pc ? rt_cvt<C>(w[v * Nhs + z * zs + p]) : C{0, 0};
+      return p < pc && R3D_W(v * Nhs + z * zs + p) ? rt_cvt<C>(w[v * Nhs + z * zs + p]) : C{0, 0};
     };
     rt_pass_s<NZ, -1, NT, RM>(d.rtz, s, W, mgW, tw, ld, sts);
     __syncthreads();
@@ -455,7 +464,9 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_zoz(Batch b) {
         const int kz = zrev[s], az = 2 * kz - nz + 1;
         // cubic cells: shell (ax^2 + ay^2 + az^2 - 3) / 8, below 2^31 up to
         // 2048 points a side
+        if (!cubic && !R3D_IN(d, ((long long)kz * ny + ky) * hx + kx, d.Nh)) continue;
         const uint32_t shell = cubic ? (uint32_t)(axy + az * az) >> 3 : kidx[kz * zs];
+        if (cubic && !R3D_IN(d, shell, (3LL * (nz - 1) * (nz - 1) - 3) / 8 + 1)) continue;
         const X *ch = chi + (size_t)shell * chis;
 #pragma unroll
         for (int o = 0; o < OS; ++o) {
@@ -515,7 +526,8 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_zoz(Batch b) {
         sts(c, z, a);
       } else {
         const int p = c % PC, v = c / PC;
-        if (p < pc) w[v * Nhs + z * zs + p] = rt_cvt<S>(a);
+        if (p < pc && R3D_W(v * Nhs + z * zs + p))
+          w[v * Nhs + z * zs + p] = rt_cvt<S>(a);
       }
     };
     rt_pass_s<NZ, 1, NT, RM>(d.rtz, s, W, mgW, tw, lds, st);
@@ -575,7 +587,9 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_inv(Batch b, int mode) {
         rt_edge<NY, RM>(
             NY ? 0 : d.rty.n, s,
             [&] {
-              auto ld = [&](int p, int y) { return rt_cvt<C>(w[y * hx + p]); };
+              auto ld = [&](int p, int y) {
+                return R3D_W(y * hx + p) ? rt_cvt<C>(w[y * hx + p]) : C{0, 0};
+              };
               rt_pass_s<NY, 1, NT, RM>(d.rty, s, hx, mghx, twy, ld, st);
             },
             [&] {
@@ -591,7 +605,8 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_inv(Batch b, int mode) {
         S a[U];
 #pragma unroll
         for (int k = 0; k < U; ++k)
-          if (e0 + k * NT < nrow * hx) a[k] = w[e0 + k * NT];
+          if (e0 + k * NT < nrow * hx && R3D_W(e0 + k * NT))
+            a[k] = w[e0 + k * NT];
 #pragma unroll
         for (int k = 0; k < U; ++k) {
           const int e = e0 + k * NT, r = rt_div(e, mghx), p = e - r * hx;
@@ -683,7 +698,8 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_inv(Batch b, int mode) {
     double s = 0;
 #pragma unroll
     for (int i = 0; i < NW; ++i) s += red[threadIdx.x][i];
-    d.partials[((size_t)v * 6 + threadIdx.x) * d.rt_icps + part] = s;
+    if (R3D_IN(d, (v * 6 + threadIdx.x) * d.rt_icps + part, 6 * d.n * d.rt_icps))
+      d.partials[((size_t)v * 6 + threadIdx.x) * d.rt_icps + part] = s;
     __threadfence();
   }
   __syncthreads();
@@ -700,10 +716,6 @@ __global__ void __launch_bounds__(NT, MINB) k_rt_inv(Batch b, int mode) {
 // the reduce alone (anderson(): mode 1), one CTA per solve
 __global__ void __launch_bounds__(kThreads) k_rt_reduce(const Desc *descs, int mode) {
   const Desc &d = descs[blockIdx.x];
-  if (d.ctl->status != RUNNING && mode == 0) {
-    if (threadIdx.x == 0) d.ctl->mix_flag = 0;
-    return;
-  }
   rt_reduce<kThreads>(d, mode, d.mixer == MIX_AN2 && d.ctl->count_left <= 0);
 }
 #endif

@@ -114,7 +114,7 @@ import rism3d as R
 assert R.LIB_PATH.endswith("_debug.so"), R.LIB_PATH
 out = {}
 for prec in ("fp64", "mixed"):
-    for xv, yz in (("1", "2"), ("4", "3"), ("4", "4"), ("2", "0")):
+    for xv, yz in (("1", "2"), ("4", "3"), ("4", "4"), ("2", "0"), ("5", "0")):
         os.environ["R3D_X_VARIANT"], os.environ["R3D_YZ_VARIANT"] = xv, yz
         s = R.RISM3D(precision=prec)
         s.initialize(%(inp)r, xvk=%(xvk)r)
