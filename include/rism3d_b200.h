@@ -183,7 +183,8 @@ int r3d_refresh_timing(const r3d_ctx *ctx, int *count, double *ms);
 
 /* Advance the solve by exactly `nsteps` iterations (graph replays, no
  * convergence polling; converged or diverged solves do no further work) and
- * return their CUDA-event time in *ms.  No counterpart in the reference: the
+ * return their CUDA-event time in *ms.  Every iteration's mix has been applied
+ * on return: t is the t of the start of the next one.  No counterpart in the reference: the
  * benchmark and batch loops use it to time iterations without host syncs. */
 int r3d_step(r3d_ctx *ctx, int nsteps, double *ms);
 
