@@ -820,9 +820,9 @@ static int plan_geo(r3d_ctx *c, Desc &d, Geo &g, bool fp64, int nsites) {
 // The variants of the per-axis iteration passes that a geometry offers.  Planning
 // them opts every kernel of theirs into large shared memory and asks for
 // occupancies, which loads the kernels: a solve on the plane passes skips it
-// (r3d_initialize of a process' first solve, this and opt-ins by length alone:
-// 96^3 mixed 110 ms against 300, 64^3 FP64 110 against 160, 144^3 mixed 128 against
-// 310).
+// (r3d_initialize of a process' first solve, with opt-ins by length and objects
+// that unpack fast: 96^3 mixed 97 ms against 300, 64^3 FP64 91 against 158, 144^3
+// mixed 107 against 303; 80 x 72 x 96 FP64, on these variants, 170 against 198).
 static void plan_variants(r3d_ctx *c, Desc &d, Geo &g, bool fp64) {
   const size_t cs = fp64 ? 16 : 8;
   const int rowsN = d.ny * d.nz;
